@@ -189,17 +189,16 @@ template <class R> __device__ __forceinline__ void forward_update(const Gas<R>& 
                                                                   R* qn, bool cons) {
   if (cons) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) qn[v] = q0[v] + tot[v] * fac;
+    for (int v = 0; v < 4; ++v) qn[v] = mad(tot[v], fac, q0[v]);
     return;
   }
   // conserved set of q0: r u, r v, r, r h - p = p/(gamma-1) + r |u|^2/2
   R qc[4];
-  R u2 = q0[0] * q0[0];
-  u2 += q0[1] * q0[1];
+  const R u2 = mad(q0[1], q0[1], q0[0] * q0[0]);
   qc[0] = q0[2] * q0[0]; qc[1] = q0[2] * q0[1]; qc[2] = q0[2];
-  qc[3] = fma(q0[3], g.gamma1, q0[2] * (R(0.5) * u2));  // one contraction, whatever the kernel
+  qc[3] = mad(q0[3], g.gamma1, q0[2] * (R(0.5) * u2));  // one contraction, whatever the kernel
 #pragma unroll
-  for (int v = 0; v < 4; ++v) qc[v] = qc[v] + tot[v] * fac;
+  for (int v = 0; v < 4; ++v) qc[v] = mad(tot[v], fac, qc[v]);
   const St<R> s1 = cons_state(g, qc);
   qn[0] = s1.u; qn[1] = s1.v; qn[2] = s1.r; qn[3] = s1.p;
 }
@@ -376,10 +375,10 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
           const C q0 = Q(v, la, lb);
           const C a0 = q0 - Q(v, la - 1, lb), a1 = Q(v, la + 1, lb) - q0;
           const C b0 = q0 - Q(v, la, lb - 1), b1 = Q(v, la, lb + 1) - q0;
-          m[2 * v] += a0 * dxi0; m[2 * v + 1] += a0 * dyi0;
-          m[2 * v] += a1 * dxi1; m[2 * v + 1] += a1 * dyi1;
-          m[2 * v] += b0 * dxj0; m[2 * v + 1] += b0 * dyj0;
-          m[2 * v] += b1 * dxj1; m[2 * v + 1] += b1 * dyj1;
+          m[2 * v] = mad(a0, dxi0, m[2 * v]); m[2 * v + 1] = mad(a0, dyi0, m[2 * v + 1]);
+          m[2 * v] = mad(a1, dxi1, m[2 * v]); m[2 * v + 1] = mad(a1, dyi1, m[2 * v + 1]);
+          m[2 * v] = mad(b0, dxj0, m[2 * v]); m[2 * v + 1] = mad(b0, dyj0, m[2 * v + 1]);
+          m[2 * v] = mad(b1, dxj1, m[2 * v]); m[2 * v + 1] = mad(b1, dyj1, m[2 * v + 1]);
         }
       }
       mstore(la, lb, m);
@@ -421,8 +420,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
         for (int v = 0; v < 4; ++v) {
           // (q_right - q_left) of the face
           const C dq = hi ? (Q(v, na, nb) - Q(v, la, lb)) : (Q(v, la, lb) - Q(v, na, nb));
-          m[2 * v] += dq * dx;
-          m[2 * v + 1] += dq * dy;
+          m[2 * v] = mad(dq, dx, m[2 * v]);
+          m[2 * v + 1] = mad(dq, dy, m[2 * v + 1]);
         }
       }
     }
@@ -435,6 +434,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
   const Gas<C> g = gas_as<C>(a.gas);
   const bool cons = a.basis != 0;  // conserved solution basis
   const int lim = LIM >= 0 ? LIM : a.limiter;
+  // the spectral radius enters the timestep, which stage 0 sets
+  const bool want_lam = a.stage == 0;
   constexpr int NFI = (TI + 1) * TJ, NFJ = TI * (TJ + 1);
   // one face: i-face kk (dir true) or j-face kk of the tile; dir is a bool, or a
   // std::integral_constant that makes the direction a compile-time constant
@@ -478,8 +479,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
             for (int v = 0; v < 4; ++v) {
               const C dq = qr[v] - ql[v];
               gc[v] = dq * idlr;
-              gl[v] = (M(2 * v, la_l, lb_l) * wlx + M(2 * v + 1, la_l, lb_l) * wly) - dq * sl;
-              gr[v] = (M(2 * v, la, lb) * wrx + M(2 * v + 1, la, lb) * wry) - dq * sr;
+              gl[v] = fma(-dq, sl, fma(M(2 * v + 1, la_l, lb_l), wly, M(2 * v, la_l, lb_l) * wlx));
+              gr[v] = fma(-dq, sr, fma(M(2 * v + 1, la, lb), wry, M(2 * v, la, lb) * wrx));
             }
             limit4x2(lim, gc, gl, gr, sL, sR);
             if constexpr (REC) {
@@ -496,8 +497,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
             }
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-              qL[v] = ql[v] + dl * sL[v];
-              qR[v] = qr[v] - dr * sR[v];
+              qL[v] = fma(dl, sL[v], ql[v]);
+              qR[v] = fma(-dr, sR[v], qr[v]);
             }
           } else {
             C ml[8], mr[8];
@@ -525,23 +526,23 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
           if constexpr (REC) {
             St<C> sL, sR;
             basis_state2(g, qL, qR, cons, sL, sR);
-            F = face_flux<C, FK>(g, nx, ny, A, sL, sR);
+            F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
             sg |= (unsigned long long)flux_bits<C, FK>(g, nx, ny, sL, sR) << SIG_FLUX_SHIFT;
           } else {
             St<C> sL, sR;
             basis_state2(g, qL, qR, cons, sL, sR);
-            F = face_flux<C, FK>(g, nx, ny, A, sL, sR);
+            F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
           }
         } else {
           if constexpr (REC) {
             St<C> sL, sR;
             basis_state2(g, ql, qr, cons, sL, sR);
-            F = face_flux<C, FK>(g, nx, ny, A, sL, sR);
+            F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
             sg |= (unsigned long long)flux_bits<C, FK>(g, nx, ny, sL, sR) << SIG_FLUX_SHIFT;
           } else {
             St<C> sL, sR;
             basis_state2(g, ql, qr, cons, sL, sR);
-            F = face_flux<C, FK>(g, nx, ny, A, sL, sR);
+            F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
           }
         }
       } else {
@@ -607,12 +608,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
           if constexpr (REC) {
             St<C> sL, sR;
             basis_state2(g, qL, qR, cons, sL, sR);
-            F = face_flux<C, FK>(g, nx, ny, A, sL, sR);
+            F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
             sg |= (unsigned long long)flux_bits<C, FK>(g, nx, ny, sL, sR) << SIG_FLUX_SHIFT;
           } else {
             St<C> sL, sR;
             basis_state2(g, qL, qR, cons, sL, sR);
-            F = face_flux<C, FK>(g, nx, ny, A, sL, sR);
+            F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
           }
         }
       }
@@ -675,7 +676,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
   if (own && a.res_out) {
 #pragma unroll
     for (int v = 0; v < 4; ++v) a.res_out[v * ncell + c] = res[v];
-    a.res_out[4 * ncell + c] = lam;
+    if (want_lam) a.res_out[4 * ncell + c] = lam;
   }
   if (a.mode == MODE_RES_MAXRATE) {
     // spectralRadius: max over cells of lambda/V (spatial/spectralRadius.h:19-48)
@@ -710,19 +711,19 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
   R tot[4] = {R(0), R(0), R(0), R(0)};
   for (int k = 0; k < a.stage; ++k)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) tot[v] += a.alpha[k] * a.res_prev[k][v * ncell + c];
+    for (int v = 0; v < 4; ++v) tot[v] = mad(a.alpha[k], a.res_prev[k][v * ncell + c], tot[v]);
 #pragma unroll
-  for (int v = 0; v < 4; ++v) tot[v] += a.alpha[a.stage] * res[v];
+  for (int v = 0; v < 4; ++v) tot[v] = mad(a.alpha[a.stage], res[v], tot[v]);
   R fac;
   if (a.mode == MODE_FUSED_GLOBAL) {
     const R dts = a.beta * R(a.info->dt);
-    fac = qdiv(dts, a.vol[c]);
+    fac = div_fast(dts, a.vol[c]);
   } else {
     // local timestep from the stage-0 spectral radius sum (eulerForwardUpdate.h:155-161)
     const R l0 = (a.stage == 0) ? lam : a.res_prev[0][4 * ncell + c];
     const R cs = a.beta * a.cfl;
     // dual time: dtau / (1 + b0 dtau / dt), the physical-time term's share of the spectral radius
-    fac = (DUAL && a.dual_src) ? cs / (l0 + a.cfl * a.vol[c] * a.dual_b0dt) : qdiv(cs, l0);
+    fac = (DUAL && a.dual_src) ? cs / (l0 + a.cfl * a.vol[c] * a.dual_b0dt) : div_fast(cs, l0);
   }
   R q0[4], qn[4];
 #pragma unroll
@@ -787,7 +788,7 @@ __device__ __forceinline__ void update0_cell(size_t c, size_t ncell, const Gas<R
     tot[v] = R(0) + alpha00 * res0[v * ncell + c];
     q[v] = q0[v * ncell + c];
   }
-  const R fac = dts / vol[c];
+  const R fac = div_fast(dts, vol[c]);
   forward_update(g, q, tot, fac, qn, cons);
 #pragma unroll
   for (int v = 0; v < 4; ++v) q_out[v * ncell + c] = qn[v];

@@ -75,6 +75,7 @@ template <class T> __host__ __device__ __forceinline__ bool isfinite(Tan<T> x) {
   using ::isfinite;
   return isfinite(x.v);
 }
+template <class T> __host__ __device__ __forceinline__ float rough(Tan<T> x) { return hc::rough<T>(x.v); }
 
 }  // namespace tg
 using tg::Tan;
