@@ -187,8 +187,7 @@ template <class R> int run_step_1d_smoothed(hc_ctx* c) {
   R* wrk = (R*)c->smooth_buf;
   R* tmp = wrk + 3 * n;
   const int ends = c->bc[0] == HC_BC_PERIODIC ? 'p' : 'a';
-  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, sizeof(unsigned long long), c->stream));
-  HC_CUDA(cudaMemsetAsync(&c->info->resnorm2, 0, sizeof(double), c->stream));
+  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
   auto out_of = [&](int s) -> R* { return (R*)((s == nst - 1) ? c->q[0] : c->q[1 + (s % 2)]); };
   for (int s = 0; s < nst; ++s) {
     Stage1DArgs<R> a = args_1d<R>(c);
@@ -226,8 +225,7 @@ template <class R> int run_step_1d(hc_ctx* c) {
   const RKTab tab = rk_table(c->cfg.rk);
   const int nst = tab.nst;
   const bool global = c->cfg.dt_mode == HC_DT_GLOBAL;
-  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, sizeof(unsigned long long), c->stream));
-  HC_CUDA(cudaMemsetAsync(&c->info->resnorm2, 0, sizeof(double), c->stream));
+  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
   auto out_of = [&](int s) -> R* { return (R*)((s == nst - 1) ? c->q[0] : c->q[1 + (s % 2)]); };
   for (int s = 0; s < nst; ++s) {
     Stage1DArgs<R> a = args_1d<R>(c);
@@ -280,8 +278,7 @@ template <class R> int run_step(hc_ctx* c) {
   auto fn = [c, euler_fn](const StageArgs<R>& a, int tile, cudaStream_t s) -> cudaError_t {
     return c->scalar ? launch_scalar_stage<R>(a, c->cfg.flux, tile, s) : euler_fn(a, tile, s);
   };
-  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, sizeof(unsigned long long), c->stream));
-  HC_CUDA(cudaMemsetAsync(&c->info->resnorm2, 0, sizeof(double), c->stream));
+  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
   auto out_of = [&](int s) -> R* { return (R*)((s == nst - 1) ? c->q[0] : c->q[1 + (s % 2)]); };
   for (int s = 0; s < nst; ++s) {
     StageArgs<R> a = base_args<R>(c);
@@ -552,9 +549,9 @@ int hc_context_create(const hc_config* cfg, hc_ctx** out) {
   c->df = cfg->precision == HC_FP64_DF;
   // measured on the 512 x 1024 O-grid (Roe, van Albada): FP64 16x16 cells on 128 threads
   // 2.9% faster than on 256 and 4.4% faster than 8x32 (four CTAs per SM instead of two
-  // overlap one another's load and barrier phases; the 544 faces fill whole warps), FP32
-  // 8x32 (3.6% faster than 16x16)
-  c->tile = c->fp32 ? TILE_8x32 : TILE_16x16_H;
+  // overlap one another's load and barrier phases; the 544 faces fill whole warps), smaller
+  // tiles on small meshes (f64_auto_tile); FP32 8x32 (3.6% faster than 16x16)
+  c->tile = c->fp32 ? TILE_8x32 : TILE_AUTO;
   c->rsz = c->fp32 ? sizeof(float) : sizeof(double);
   cudaError_t e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
   if (e == cudaSuccess) {

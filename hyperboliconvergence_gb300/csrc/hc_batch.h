@@ -82,9 +82,7 @@ template <class R> BatchArgs<R> batch_args(hc_batch* b) {
 
 // maxrate and resnorm2 of every instance's StepInfo (strided)
 inline int zero_step_words(hc_batch* b) {
-  HC_CUDA(cudaMemset2DAsync(&b->info[0].maxrate, sizeof(StepInfo), 0, sizeof(unsigned long long), b->ninst,
-                            b->stream));
-  HC_CUDA(cudaMemset2DAsync(&b->info[0].resnorm2, sizeof(StepInfo), 0, sizeof(double), b->ninst, b->stream));
+  HC_CUDA(cudaMemset2DAsync(&b->info[0].maxrate, sizeof(StepInfo), 0, kStepWords, b->ninst, b->stream));
   return HC_OK;
 }
 

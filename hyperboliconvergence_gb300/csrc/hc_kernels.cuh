@@ -31,12 +31,14 @@ enum FaceField { F_NX = 0, F_NY, F_A, F_DL, F_DR, F_IDLR, F_WLX, F_WLY, F_SL, F_
 // Per-step scalars shared by the kernels of one RK step (device memory).
 struct StepInfo {
   unsigned long long maxrate;  // max over cells of lambda/V as the bit pattern of a positive double
+  double resnorm2;             // sum over cells of the stage-0 density residual squared
   double dt;                   // global timestep of the current step
   double t;                    // accumulated time
   int status;                  // 0 ok, 1 non-physical state produced
   int bad_cell;                // first cell found non-physical
-  double resnorm2;             // sum over cells of the stage-0 density residual squared
 };
+// maxrate and resnorm2 lie side by side: one memset clears both at the start of a step
+constexpr size_t kStepWords = sizeof(unsigned long long) + sizeof(double);
 
 // Status codes of the device-side checks
 enum { ST_OK = 0, ST_NONPHYSICAL = 1, ST_TIMEOUT = 2 };
@@ -256,8 +258,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
   const C* cfi = same ? reinterpret_cast<const C*>(a.fi) : reinterpret_cast<const C*>(a.fic);
   const C* cfj = same ? reinterpret_cast<const C*>(a.fj) : reinterpret_cast<const C*>(a.fjc);
   constexpr int QI = SM::QI, QJ = SM::QJ, MI = SM::MI, MJ = SM::MJ;
-  constexpr int NT = NTH;  // threads of the block: TI*TJ, or a divisor of it (several cells per thread)
-  static_assert((TI * TJ) % NTH == 0 && NTH % 32 == 0, "threads must divide the tile's cells in whole warps");
+  constexpr int NT = NTH;  // threads of the block: TI*TJ, a divisor of it (several cells per thread) or more
+  static_assert(((TI * TJ) % NTH == 0 || NTH > TI * TJ) && (TI * TJ) % 32 == 0 && NTH % 32 == 0,
+                "the tile's cells take whole warps");
   const int ni = a.ni, nj = a.nj;
   const size_t ncell = size_t(ni) * nj;
   const int i0 = bi * TI, j0 = bj * TJ;

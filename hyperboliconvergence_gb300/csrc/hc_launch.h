@@ -7,6 +7,7 @@
 #include "hc_tma.h"
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 #include <vector>
 
@@ -14,7 +15,39 @@ namespace hc {
 
 // Tile shapes the stage kernel is built for (cells along i x cells along j).
 // TILE_16x16_H: 16 x 16 cells run by 128 threads (two cells a thread in the update)
-enum TileShape { TILE_8x32 = 0, TILE_4x32 = 1, TILE_16x16 = 2, TILE_16x16_H = 3, TILE_COUNT = 4 };
+// TILE_AUTO (FP64 single-mesh default): 16x16_H, 8x8 or 4x8 by the mesh's size (f64_auto_tile)
+enum TileShape { TILE_8x32 = 0, TILE_4x32 = 1, TILE_16x16 = 2, TILE_16x16_H = 3, TILE_COUNT = 4, TILE_AUTO = 5,
+                 TILE_8x8 = 6, TILE_4x8 = 7 };
+
+// Tile of an FP64 stage launch.  The stage takes as long as its busiest SM, whose time is the
+// FP64 instructions of its tiles: an SM starts one per 19 cycles and each of its four
+// sub-partitions one per 64 (measured), whatever the number of active lanes.  So a tile costs
+// its warps of faces (230 instructions each), of gradient cells (48) and of cells (60), and
+// the shape whose fullest SM is done first wins: small tiles spread a small mesh over the 152
+// SMs, large ones repeat fewer faces and gradients.  Measured (Roe, ms per ssp34 step; always
+// 16x16 against this rule): 40 x 40 0.263 -> 0.082, 128 x 128 0.260 -> 0.140, 200 x 200 0.394
+// -> 0.291; SLAU 300 x 401 0.845 -> 0.649; 256 x 512 and larger stay on 16x16.
+inline double f64_tile_cost(int ni, int nj, int ti, int tj, int sms) {
+  const long long tiles = (long long)((ni + ti - 1) / ti) * ((nj + tj - 1) / tj);
+  const double k = double((tiles + sms - 1) / sms);
+  auto pass = [k](int items, int instr) {  // warps of one phase, dealt to four sub-partitions
+    const double w = k * ((items + 31) / 32);
+    return instr * (w > 16 ? 19.0 * w : 64.0 * std::ceil(w / 4));
+  };
+  return pass((ti + 1) * tj + ti * (tj + 1), 230) + pass((ti + 2) * (tj + 2), 48) + pass(ti * tj, 60);
+}
+inline int f64_auto_tile(int ni, int nj) {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 152;
+  }();
+  const double c16 = f64_tile_cost(ni, nj, 16, 16, sms), c8 = f64_tile_cost(ni, nj, 8, 8, sms),
+               c4 = f64_tile_cost(ni, nj, 4, 8, sms);
+  if (c16 <= c8 && c16 <= c4) return TILE_16x16_H;
+  return c8 <= c4 ? TILE_8x8 : TILE_4x8;
+}
 
 template <class R, int FK> cudaError_t launch_stage(const StageArgs<R>& a, int tile, cudaStream_t s);
 template <class R, int FK> cudaError_t prepare_stage();
@@ -182,6 +215,19 @@ inline void tile_dims(int tile, int* ti, int* tj) {
     }                                                                                                    \
     if constexpr (std::is_same<R, float>::value) {                                                       \
       if ((tile == TILE_8x32 || tile < 0 || tile >= TILE_COUNT) && go_fixed_lim(a, s)) return cudaGetLastError(); \
+    }                                                                                                    \
+    if constexpr (std::is_same<R, double>::value) {                                                      \
+      if (tile == TILE_AUTO) tile = f64_auto_tile(a.ni, a.nj);                                           \
+      if (tile == TILE_8x8) {                                                                            \
+        const dim3 grid((a.nj + 7) / 8, (a.ni + 7) / 8);                                                 \
+        stage_kernel<8, 8, R, FK, R, 160><<<grid, 160, StageSmem<8, 8, R>::bytes, s>>>(a);               \
+        return cudaGetLastError();                                                                       \
+      }                                                                                                  \
+      if (tile == TILE_4x8) {                                                                            \
+        const dim3 grid((a.nj + 7) / 8, (a.ni + 3) / 4);                                                 \
+        stage_kernel<4, 8, R, FK, R, 96><<<grid, 96, StageSmem<4, 8, R>::bytes, s>>>(a);                 \
+        return cudaGetLastError();                                                                       \
+      }                                                                                                  \
     }                                                                                                    \
     if (tile == TILE_4x32) go<R, 4, 32>(a, s);                                                           \
     else if (tile == TILE_16x16) go<R, 16, 16>(a, s);                                                    \
