@@ -55,6 +55,8 @@ void free_buffers(hc_ctx* c) {
     if (c->fj) cudaFree(c->fj);
     if (c->vol) cudaFree(c->vol);
   }
+  if (c->pk) cudaFree(c->pk);
+  c->pk = nullptr;
   if (c->fic) cudaFree(c->fic);
   if (c->fjc) cudaFree(c->fjc);
   c->nodes = c->cx = c->cy = c->xm = c->fi64 = c->fj64 = c->vol64 = c->staging = nullptr;
@@ -110,6 +112,10 @@ int build_geometry(hc_ctx* c) {
     convert_kernel<float><<<1024, 256, 0, c->stream>>>(c->fj64, (float*)c->fj, size_t(FREC) * nfj);
     convert_kernel<float><<<1024, 256, 0, c->stream>>>(c->vol64, (float*)c->vol, n);
     c->launches += 3;
+    if (c->pk) {
+      HC_CUDA(pack_strips(c->fi64, c->fj64, c->vol64, ni, nj, c->bc, c->pk, c->stream));
+      c->launches += 1;
+    }
   }
   if (c->df) {
     convert_kernel<df64><<<1024, 256, 0, c->stream>>>(c->fi64, (df64*)c->fic, size_t(FREC) * nfi);
@@ -623,6 +629,7 @@ int hc_mesh_upload(hc_ctx* c, int ni, int nj, const double* nodes_xy) {
     HC_CUDA(cudaMalloc(&c->fi, FREC * nfi * sizeof(float)));
     HC_CUDA(cudaMalloc(&c->fj, FREC * nfj * sizeof(float)));
     HC_CUDA(cudaMalloc(&c->vol, n * sizeof(float)));
+    if (!c->scalar) HC_CUDA(cudaMalloc(&c->pk, strip_floats(ni, nj) * sizeof(float)));
     HC_CUDA(cudaMalloc(&c->staging, 5 * n * sizeof(double)));
   } else {
     c->fi = c->fi64; c->fj = c->fj64; c->vol = c->vol64;

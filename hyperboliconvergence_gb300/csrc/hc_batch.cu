@@ -2,7 +2,6 @@
 // one persistent launch per RK stage over a shared work list of tiles, with
 // CUDA-graph capture and a schedule autotuner.
 #include "hc_batch.h"
-#include "hc_tma.h"
 
 #include <algorithm>
 #include <cstring>
@@ -29,7 +28,7 @@ void free_all(hc_batch* b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   b->graph_exec = nullptr; b->graph = nullptr;
   void* ptrs[] = {b->nodes, b->cx, b->cy, b->xm, b->vol64, b->fi64, b->fj64, b->gref, b->q[0], b->q[1], b->q[2],
-                  b->res[0], b->res[1], b->res[2], b->staging, b->info, b->inst_d, b->order_d, b->tma_maps};
+                  b->res[0], b->res[1], b->res[2], b->staging, b->info, b->inst_d, b->order_d, b->pk, b->strip_order_d};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (b->fp32) {
@@ -57,6 +56,7 @@ int build_worklist(hc_batch* b) {
     in.tiles_i = (in.ni + ti - 1) / ti;
     in.tiles_j = (in.nj + tj - 1) / tj;
     in.cell = b->cell_off[k]; in.fi = b->fi_off[k]; in.fj = b->fj_off[k];
+    in.pk = b->pk ? b->pk_off[k] : 0;
     if (in.tiles_i * in.tiles_j > 0xffff) return fail(HC_ERR_UNSUPPORTED, "instance has more than 65535 tiles");
   }
   for (int k : perm) {
@@ -71,6 +71,24 @@ int build_worklist(hc_batch* b) {
     b->nwork_cap = b->nwork;
   }
   HC_CUDA(cudaMemcpyAsync(b->order_d, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+  std::vector<int> strips;
+  if (b->pk) {
+    b->strip_rows = strip_run_rows(b->ninst, [&](int k) { return b->ni[k]; }, [&](int k) { return b->nj[k]; }, b->sms);
+    for (int k : perm) {
+      const int nt = strip_count(b->nj[k]) * ((b->ni[k] + b->strip_rows - 1) / b->strip_rows);
+      if (nt > 0xffff) return fail(HC_ERR_UNSUPPORTED, "instance has more than 65535 strips");
+      for (int t = 0; t < nt; ++t) strips.push_back((k << 16) | t);
+    }
+    b->strip_work = int(strips.size());
+    if (b->strip_work > b->strip_cap) {
+      if (b->strip_order_d) cudaFree(b->strip_order_d);
+      b->strip_order_d = nullptr;
+      HC_CUDA(cudaMalloc(&b->strip_order_d, strips.size() * sizeof(int)));
+      b->strip_cap = b->strip_work;
+    }
+    HC_CUDA(cudaMemcpyAsync(b->strip_order_d, strips.data(), strips.size() * sizeof(int), cudaMemcpyHostToDevice,
+                            b->stream));
+  }
   HC_CUDA(cudaMemcpyAsync(b->inst_d, b->inst_h.data(), b->inst_h.size() * sizeof(BatchInst), cudaMemcpyHostToDevice,
                           b->stream));
   HC_CUDA(cudaStreamSynchronize(b->stream));
@@ -78,43 +96,6 @@ int build_worklist(hc_batch* b) {
 }
 
 
-
-// Tensor maps of an FP32 Euler batch (hc_tma.h): per instance, the three state pools' slices
-// (4 planes of ni x nj) and its i-face records; none when any instance's rows are not a
-// multiple of 16 bytes or a slice is not 16-byte aligned (the batch then keeps plain loads).
-int build_tma_maps(hc_batch* b) {
-  if (!b->fp32 || b->scalar) return HC_OK;
-  const int n = b->ninst;
-  std::vector<CUtensorMap> maps(size_t(4) * n);
-  for (int k = 0; k < n; ++k) {
-    StageArgs<float> a{};
-    a.ni = b->ni[k];
-    a.nj = b->nj[k];
-    a.fi = (const float*)b->fi + (long long)FREC * b->fi_off[k];
-    for (int buf = 0; buf < 3; ++buf) {
-      a.q = (const float*)b->q[buf] + 4 * b->cell_off[k];
-      CUtensorMap tfi;
-      if (!stage_tma_maps(a, &maps[size_t(buf) * n + k], &tfi)) return HC_OK;
-      if (buf == 0) maps[size_t(3) * n + k] = tfi;
-    }
-  }
-  HC_CUDA(cudaMalloc((void**)&b->tma_maps, maps.size() * sizeof(CUtensorMap)));
-  HC_CUDA(cudaMemcpy(b->tma_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
-  return HC_OK;
-}
-
-// the maps of stage input pool q (one of b->q[0..2]) and of the records, or nulls
-template <class R> void tma_args(hc_batch* b, BatchArgs<R>& a) {
-  a.tmaps_q = a.tmaps_fi = nullptr;
-  if constexpr (std::is_same<R, float>::value) {
-    if (!b->tma_maps || b->sched.tile != HC_TILE_8x32) return;
-    for (int buf = 0; buf < 3; ++buf)
-      if (a.q == (const R*)b->q[buf]) {
-        a.tmaps_q = b->tma_maps + size_t(buf) * b->ninst;
-        a.tmaps_fi = b->tma_maps + size_t(3) * b->ninst;
-      }
-  }
-}
 
 template <class R> int persistent_step(hc_batch* b) {
   const RKTab tab = rk_table(b->cfg.rk);
@@ -130,7 +111,8 @@ template <class R> int persistent_step(hc_batch* b) {
   for (int s = 0; s < nst; ++s) {
     BatchArgs<R> a = batch_args<R>(b);
     a.q = (s == 0) ? (const R*)b->q[0] : out_of(s - 1);
-    tma_args(b, a);
+    // the schedule's CTAs of 256 threads are two of the strip kernel's blocks each
+    a.strip_grid = std::min(a.strip_grid, b->sms * 2 * std::max(1, b->sched.ctas_per_sm));
     a.stage = s;
     a.beta = R(tab.beta[s]);
     for (int k = 0; k <= s; ++k) a.alpha[k] = R(tab.alpha[s][k]);
@@ -185,6 +167,7 @@ template <class R> int per_instance_step(hc_batch* b) {
     base.fi = (const R*)b->fi + (long long)FREC * b->fi_off[k];
     base.fj = (const R*)b->fj + (long long)FREC * b->fj_off[k];
     base.vol = (const R*)b->vol + b->cell_off[k];
+    base.pk = b->pk ? b->pk + b->pk_off[k] : nullptr;
     base.q0 = qp(0);
     base.info = b->info + k;
     base.cfl = R(b->cfg.cfl);
@@ -298,6 +281,7 @@ int hc_batch_create(const hc_config* cfg, int ninst, const int* ni, const int* n
     b->fi_off.push_back(b->nfi); b->nfi += size_t(ni[k] + 1) * nj[k];
     b->fj_off.push_back(b->nfj); b->nfj += size_t(ni[k]) * (nj[k] + 1);
     b->node_off.push_back(b->nnode); b->nnode += size_t(ni[k] + 1) * (nj[k] + 1) * 2;
+    b->pk_off.push_back((long long)b->npk); b->npk += strip_floats(ni[k], nj[k]);
     maxcell = std::max(maxcell, b->icells(k));
     for (int s = 0; s < 4; ++s) {
       b->gref_off.push_back(b->ngref);
@@ -324,6 +308,7 @@ int hc_batch_create(const hc_config* cfg, int ninst, const int* ni, const int* n
     e = A(&b->fi, FREC * b->nfi * 4);
     if (e == cudaSuccess) e = A(&b->fj, FREC * b->nfj * 4);
     if (e == cudaSuccess) e = A(&b->vol, b->ncell * 4);
+    if (e == cudaSuccess && !scalar) e = A((void**)&b->pk, b->npk * 4);
   } else if (e == cudaSuccess) {
     b->fi = b->fi64; b->fj = b->fj64; b->vol = b->vol64;
   }
@@ -338,6 +323,10 @@ int hc_batch_create(const hc_config* cfg, int ninst, const int* ni, const int* n
                         b->fj64 + FREC * b->fj_off[k]};
     // the xm pool is laid out per instance as 3 planes of its own cell count
     b->launches += enqueue_geometry(g, ni[k], nj[k], bc + 4 * k, b->stream);
+    if (b->pk && e == cudaSuccess) {
+      e = pack_strips(g.fi, g.fj, g.vol, ni[k], nj[k], bc + 4 * k, b->pk + b->pk_off[k], b->stream);
+      b->launches += 1;
+    }
     for (int s = 0; s < 4; ++s) {
       const int t = bc[4 * k + s];
       if (t == HC_BC_PERIODIC || t == HC_BC_WALL || !ref || !ref[4 * k + s]) continue;
@@ -361,7 +350,6 @@ int hc_batch_create(const hc_config* cfg, int ninst, const int* ni, const int* n
   }
   if (e != cudaSuccess) return bail(fail(HC_ERR_CUDA, std::string("batch set-up: ") + cudaGetErrorString(e)));
   if (int st = build_worklist(b)) return bail(st);
-  if (int st = build_tma_maps(b)) return bail(st);
   *out = b;
   return HC_OK;
 }

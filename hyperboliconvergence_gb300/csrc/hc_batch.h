@@ -4,6 +4,7 @@
 
 #include "hc_host.h"
 
+#include <algorithm>
 #include <vector>
 
 struct hc_batch {
@@ -31,10 +32,13 @@ struct hc_batch {
   double* staging = nullptr;
   hc::StepInfo* info = nullptr;
   hc::BatchInst* inst_d = nullptr;
-  // FP32 Euler batches: per-instance tensor maps of the three state pools and of the i-face
-  // records ([4][ninst], device memory) for the TMA-staged 8x32 tile; null where a mesh's rows
-  // are not a multiple of 16 bytes
-  CUtensorMap* tma_maps = nullptr;
+  // FP32 Euler batches: the strip kernel's packed records (hc_stage_warp.cuh), its work list
+  // and rows per run
+  float* pk = nullptr;
+  std::vector<long long> pk_off;
+  size_t npk = 0;
+  int* strip_order_d = nullptr;
+  int strip_work = 0, strip_rows = 0, strip_cap = 0;
   int* order_d = nullptr;
   int nwork = 0, nwork_cap = 0;
   std::vector<hc::BatchInst> inst_h;
@@ -77,6 +81,12 @@ template <class R> BatchArgs<R> batch_args(hc_batch* b) {
   a.gref = (const R*)b->gref;
   a.cfl = R(b->cfg.cfl);
   a.info = b->info;
+  a.pk = b->pk;
+  a.strip_order = b->strip_order_d;
+  a.strip_work = b->strip_work;
+  a.strip_rows = b->strip_rows;
+  // every SM's resident blocks (four of 128 threads)
+  a.strip_grid = std::max(1, std::min((b->strip_work + kStripWarps - 1) / kStripWarps, b->sms * 4));
   return a;
 }
 

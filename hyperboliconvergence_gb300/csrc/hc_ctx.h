@@ -24,7 +24,7 @@ struct hc_ctx {
   unsigned fixes = 0;                               // HC_FIX_* corrections (hc_set_corrections)
   int adj_tapes = -1;                               // adjoint stage tapes (hc_set_adjoint_tapes); -1 auto
   int stall_copy = 0;                               // test hook (hc_inject_stalled_copy)
-  int staged_loads = 1;                             // TMA-staged FP32 tile loads (hc_set_staged_loads)
+  int staged_loads = 1;                             // bulk-copied FP32 strip records (hc_set_staged_loads)
   // the forward sweep recorded by hc_adjoint_record for hc_adjoint_reverse (owned here,
   // released by the reverse sweep, the next record, a mesh upload or destroy)
   void* adj_tape = nullptr;
@@ -53,6 +53,7 @@ struct hc_ctx {
   void* fic = nullptr;  // face records as double-float (HC_FP64_DF)
   void* fjc = nullptr;
   void* vol = nullptr;
+  float* pk = nullptr;  // FP32 Euler: the face records in the strip kernel's layout
   void* q[3] = {nullptr, nullptr, nullptr};
   void* res[4] = {nullptr, nullptr, nullptr, nullptr};
   void* gref[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -82,6 +83,7 @@ template <class R> StageArgs<R> base_args(hc_ctx* c) {
   a.dual_b0dt = R(c->dual_b0dt);
   a.fi = (const R*)c->fi; a.fj = (const R*)c->fj; a.vol = (const R*)c->vol;
   a.fic = c->fic; a.fjc = c->fjc;
+  a.pk = c->pk;
   for (int k = 0; k < 4; ++k) a.gref[k] = (const R*)c->gref[k];
   a.q0 = (const R*)c->q[0];
   a.info = c->info;

@@ -17,8 +17,6 @@
 
 #include "hc_physics.cuh"
 
-#include <cuda.h>  // CUtensorMap (the tensor-map type of the TMA-staged FP32 stage kernel)
-
 #include <cstdint>
 #include <type_traits>
 
@@ -74,9 +72,10 @@ template <class R> struct StageArgs {
   // dual_src, Q the conserved set, dual_src (4 planes) the earlier time levels' terms
   const R* dual_src;
   R dual_g0, dual_b0dt;
-  int stall_copy;  // test hook (hc_inject_stalled_copy): the TMA-staged tile's records barrier
-                   // expects 16 bytes its copy never delivers, so the bounded wait runs out
-  int plain_loads; // host side: 1 keeps the FP32 launch on the plain-load kernel (hc_set_staged_loads)
+  const float* pk; // FP32: the face records in the strip kernel's layout (hc_stage_warp.cuh), or null
+  int stall_copy;  // test hook (hc_inject_stalled_copy): a strip's barrier expects 16 bytes its
+                   // copy never delivers, so the bounded wait runs out
+  int plain_loads; // 1: the strip kernel copies its records with plain loads (hc_set_staged_loads)
 };
 
 // Branch signature of one face (recording kernels): bits 0-15 the limiter pieces of
@@ -93,7 +92,7 @@ template <class R> __global__ void convert_kernel(const double* __restrict__ a, 
 }
 
 // ---------------------------------------------------------------- stage kernel
-// ---- TMA and mbarrier primitives (inline PTX) of the TMA-staged FP32 stage kernel
+// ---- bulk-copy barrier primitives (inline PTX) of the FP32 strip kernel (hc_stage_warp.cuh)
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -102,41 +101,14 @@ __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// a 3D box of the tensor map at (x, y, z) into shared memory, completing on bar
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-      "[%5];\n" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// wait for phase 0 of bar for at most one second: a copy that never lands marks the step
-// ST_TIMEOUT (the host returns HC_ERR_TIMEOUT) instead of hanging the GPU
+// a copy is waited for at most this long: one that never lands marks the step ST_TIMEOUT (the
+// host returns HC_ERR_TIMEOUT) instead of hanging the GPU
 constexpr unsigned long long kCopyWaitNs = 1000000000ull;
-__device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, StepInfo* info) {
-  if (mbar_try_wait(bar, 0)) return;
-  const unsigned long long t0 = globaltimer_ns();
-  while (!mbar_try_wait(bar, 0)) {
-    if (globaltimer_ns() - t0 > kCopyWaitNs) {
-      atomicCAS(&info->status, ST_OK, ST_TIMEOUT);
-      return;
-    }
-  }
-}
 
 template <int TI, int TJ, class R> struct StageSmem {
   static constexpr int QI = TI + 4, QJ = TJ + 4;   // state tile with a 2-cell halo
@@ -146,22 +118,6 @@ template <int TI, int TJ, class R> struct StageSmem {
   static constexpr size_t fi_elems = size_t(5) * (TI + 1) * TJ;
   static constexpr size_t fj_elems = size_t(5) * TI * (TJ + 1);
   static constexpr size_t bytes = (q_elems + m_elems + fi_elems + fj_elems) * sizeof(R);
-};
-
-// Shared memory of the TMA-staged tile (FP32 or FP64): the state tile as the tensor copy lands
-// it (rows of TJ + 8 values from column j0 - 4, so that each copy starts on a 16-byte
-// boundary), the qmetric tile, the i-face records' first TMA_FIELDS fields (each face's fluxes
-// later overwrite the first five fields of its own record), the j-face fluxes.
-constexpr int TMA_FIELDS = 12;  // F_NX..F_SR: the fields the face phase reads
-template <int TI, int TJ, class C = float> struct StageSmemTma {
-  static constexpr int QI = TI + 4, QJ = TJ + 8;
-  static constexpr size_t q_elems = size_t(4) * QI * QJ;
-  static constexpr size_t m_elems = size_t(8) * (TI + 2) * (TJ + 2);
-  static constexpr size_t ri_elems = size_t(TMA_FIELDS) * (TI + 1) * TJ;
-  static constexpr size_t fj_elems = size_t(5) * TI * (TJ + 1);
-  static constexpr size_t ri_offset = (q_elems + m_elems) * sizeof(C);
-  static constexpr size_t bytes = (q_elems + m_elems + ri_elems + fj_elems) * sizeof(C);
-  static_assert(ri_offset % 128 == 0, "the i-face records' tensor copy lands on a 128-byte boundary");
 };
 
 __device__ __forceinline__ int wrapi(int a, int n) {
@@ -239,22 +195,15 @@ template <class C, class R> __device__ __forceinline__ Gas<C> gas_as(const Gas<R
 // terms are honoured (the batched instantiations, which have none, compile without them).
 // LIM >= 0: the limiter is that compile-time constant (a.limiter must equal it), so its
 // selection folds away; -1: a.limiter chosen at run time.
-// TMA: the FP32 tile whose state tile (interior tiles) and i-face records arrive by tensor
-// copies (tq, tfi; bars two mbarriers in shared memory), see stage_kernel_tma.
 template <int TI, int TJ, class R, int FK, class C = R, bool REC = false, bool DUAL = true, int NTH = TI * TJ,
-          int LIM = -1, bool TMA = false>
-__device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj, unsigned char* smem_raw,
-                                           const CUtensorMap* tq = nullptr, const CUtensorMap* tfi = nullptr,
-                                           uint64_t* bars = nullptr) {
+          int LIM = -1>
+__device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj, unsigned char* smem_raw) {
   constexpr bool same = std::is_same<C, R>::value;
   using SM = StageSmem<TI, TJ, C>;
-  static_assert(!TMA || std::is_same<C, R>::value, "the TMA-staged tile computes in its storage type");
-  constexpr int QJT = TMA ? TJ + 8 : SM::QJ;  // row length of the state tile in shared memory
-  constexpr int QSH = TMA ? 2 : 0;            // its column shift (the halo's column 0 at QSH)
   C* sq = reinterpret_cast<C*>(smem_raw);
-  C* sm = sq + size_t(4) * SM::QI * QJT;
+  C* sm = sq + SM::q_elems;
   C* sfi = sm + SM::m_elems;
-  C* sfj = sfi + (TMA ? size_t(TMA_FIELDS) * (TI + 1) * TJ : SM::fi_elems);
+  C* sfj = sfi + SM::fi_elems;
   const C* cfi = same ? reinterpret_cast<const C*>(a.fi) : reinterpret_cast<const C*>(a.fic);
   const C* cfj = same ? reinterpret_cast<const C*>(a.fj) : reinterpret_cast<const C*>(a.fjc);
   constexpr int QI = SM::QI, QJ = SM::QJ, MI = SM::MI, MJ = SM::MJ;
@@ -273,44 +222,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
   // phases 1-2 (uniform per block).  FP32 only: the FP64 stage is bound by its FP64 pipe
   // and gains nothing from fewer integer instructions.  Same sums in the same order.
   const bool interior =
-      (std::is_same<C, float>::value || TMA) && i0 >= 2 && i0 + TI + 2 <= ni && j0 >= 2 && j0 + TJ + 2 <= nj;
-  // TMA: one thread arms the two barriers and issues the tensor copies -- the interior tile's
-  // state (4 planes x (TI + 4) rows x (TJ + 8) columns from (i0 - 2, j0 - 4); columns past the
-  // mesh read zeros and are never used) and the i-face records (TMA_FIELDS fields x (TI + 1)
-  // rows x TJ columns from (i0, j0); rows or columns past the mesh belong to no valid face);
-  // they land while the threads run the halo and qmetric phases
-  bool tma = false;
-  if constexpr (TMA) {
-    tma = tq != nullptr && tfi != nullptr && (smem_u32(sq) % 128u) == 0 && (smem_u32(sfi) % 128u) == 0;
-    if (tma) {
-      if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        mbar_fence_init();
-      }
-      __syncthreads();
-      if (tid == 0) {
-        // the block's earlier accesses to this shared memory (a persistent CTA's previous
-        // work item) before the tensor copies overwrite it
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        if (interior) {
-          mbar_expect_tx(&bars[0], unsigned(4 * QI * QJT * sizeof(C)));
-          tma_load_3d(sq, tq, j0 - 4, i0 - 2, 0, &bars[0]);
-        }
-        mbar_expect_tx(&bars[1], unsigned(TMA_FIELDS * (TI + 1) * TJ * sizeof(C)) + (a.stall_copy ? 16u : 0u));
-        tma_load_3d(sfi, tfi, j0, i0, 0, &bars[1]);
-      }
-    }
-  }
-  if (tma && interior) {
-    mbar_wait_bounded(&bars[0], a.info);
-  } else if (interior) {
+      std::is_same<C, float>::value && i0 >= 2 && i0 + TI + 2 <= ni && j0 >= 2 && j0 + TJ + 2 <= nj;
+  if (interior) {
     const R* qb = a.q + (size_t(i0 - 2) * nj + (j0 - 2));
     for (int k = tid; k < QI * QJ; k += NT) {
       const int la = k / QJ, lb = k % QJ;
       const size_t c = size_t(la) * nj + lb;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sq[(v * QI + la) * QJT + lb + QSH] = cvt<C>(qb[v * ncell + c]);
+      for (int v = 0; v < 4; ++v) sq[(v * QI + la) * QJ + lb] = cvt<C>(qb[v * ncell + c]);
     }
   } else {
     for (int k = tid; k < QI * QJ; k += NT) {
@@ -321,12 +240,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
       if (gj < 0 || gj >= nj) { if (per_j) gj = wrapi(gj, nj); else ok = false; }
       const size_t c = size_t(gi) * nj + gj;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sq[(v * QI + la) * QJT + lb + QSH] = ok ? cvt<C>(a.q[v * ncell + c]) : C(0);
+      for (int v = 0; v < 4; ++v) sq[(v * QI + la) * QJ + lb] = ok ? cvt<C>(a.q[v * ncell + c]) : C(0);
     }
   }
   __syncthreads();
 
-  auto Q = [&](int v, int la, int lb) -> C { return sq[(v * QI + la + 2) * QJT + lb + 2 + QSH]; };  // tile coords
+  auto Q = [&](int v, int la, int lb) -> C { return sq[(v * QI + la + 2) * QJ + lb + 2]; };  // tile coords
   // the qmetric tile: FP32 keeps a cell's eight values as two float4 (the gradients of
   // variables 0-1, then 2-3), so that a face reads a cell's eight in two vector loads;
   // the other types keep one plane per value
@@ -430,7 +349,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
     }
     mstore(la, lb, m);
   }
-  if (tma) mbar_wait_bounded(&bars[1], a.info);
   __syncthreads();
 
   // ---- phase 3: face fluxes (i-faces then j-faces of the tile, each once)
@@ -455,12 +373,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
       const C* rec = idir ? cfi : cfj;
       const int nf = idir ? nfi : nfj;
       const int fidx = idir ? gi * nj + gj : gi * (nj + 1) + gj;
-      auto rd = [&](int fld) -> C {
-        if constexpr (TMA) {
-          if (idir && tma) return sfi[fld * NFI + la * TJ + lb];  // the tensor-copied i-face records
-        }
-        return rec[size_t(fld) * nf + fidx];
-      };
+      auto rd = [&](int fld) -> C { return rec[size_t(fld) * nf + fidx]; };
       const C nx = rd(F_NX), ny = rd(F_NY), A = rd(F_A);
       const int lo = idir ? gi : gj, nalong = idir ? ni : nj;
       const int side = idir ? (lo == 0 ? 0 : 1) : (lo == 0 ? 2 : 3);
@@ -756,21 +669,6 @@ __global__ void __launch_bounds__(NT, (StageResidency<R, C, NT>::value))
   stage_tile<TI, TJ, R, FK, C, false, true, NT, LIM>(a, blockIdx.y, blockIdx.x, smem_raw);
 }
 
-// The FP32 8x32 tile with its loads staged by the Tensor Memory Accelerator: the interior
-// tile's state and every tile's i-face records arrive by cp.async.bulk.tensor copies on
-// mbarriers, issued by one thread at the start, while the threads load the halo of edge
-// tiles and form the qmetric; the j-face records and the earlier stages' residuals stay
-// plain loads (the j-face planes' row pitch, (nj + 1) values, is not a multiple of 16 bytes).
-// The tensor maps are kernel parameters (encoded per launch by the launcher, hc_tma.h).
-template <int TI, int TJ, class R, int FK, int LIM, int NT = TI * TJ>
-__global__ void __launch_bounds__(NT, (StageResidency<R, R, NT>::value))
-    stage_kernel_tma(const StageArgs<R> a, const __grid_constant__ CUtensorMap tq,
-                     const __grid_constant__ CUtensorMap tfi) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + StageSmemTma<TI, TJ, R>::bytes);
-  stage_tile<TI, TJ, R, FK, R, false, true, NT, LIM, true>(a, blockIdx.y, blockIdx.x, smem_raw, &tq, &tfi, bars);
-}
-
 // the recording variant (a diagnostic, not on the stepping path): the same tile with
 // each face's branch signature written out
 template <int TI, int TJ, class R, int FK, class C = R>
@@ -832,6 +730,7 @@ struct BatchInst {
   long long cell;        // offset of the instance's cells in the cell pools
   long long fi, fj;      // offsets of its i-/j-face records (records, not values)
   long long gref[4];     // offsets of its ghost-reference planes (values)
+  long long pk;          // offset of its packed records (values; FP32 Euler batches)
 };
 
 template <class R> struct BatchArgs {
@@ -855,10 +754,11 @@ template <class R> struct BatchArgs {
   R beta, cfl;
   StepInfo* info;          // one per instance
   int basis;               // solution basis: 0 primitive, 1 conserved
-  // FP32 8x32 batches: per-instance tensor maps of the stage input buffer and of the i-face
-  // records (device memory), or null (plain loads)
-  const CUtensorMap* tmaps_q;
-  const CUtensorMap* tmaps_fi;
+  // FP32 Euler batches: the packed records of the strip kernel (hc_stage_warp.cuh), its work
+  // list and rows per run, and its grid
+  const float* pk;
+  const int* strip_order;
+  int strip_work, strip_rows, strip_grid;
 };
 
 template <class R> __device__ __forceinline__ StageArgs<R> instance_args(const BatchArgs<R>& b, int k) {
@@ -876,6 +776,7 @@ template <class R> __device__ __forceinline__ StageArgs<R> instance_args(const B
   a.dual_b0dt = R(0);
   a.stall_copy = 0;
   a.plain_loads = 0;
+  a.pk = b.pk ? b.pk + in.pk : nullptr;
   a.fic = a.fjc = nullptr;  // batches compute in their storage type
   const long long n = (long long)in.ni * in.nj;
   const long long off4 = 4 * in.cell, off5 = 5 * in.cell;
@@ -927,34 +828,6 @@ __global__ void __launch_bounds__(TI * TJ, (BatchResidency<R, TI * TJ>::value))
     }
     __syncthreads();
     stage_tile<TI, TJ, R, FK, R, false, false, TI * TJ, LIM>(sa, tile_ij[0], tile_ij[1], smem_raw);
-  }
-}
-
-// The persistent batch kernel with the TMA-staged FP32 8x32 tile (stage_kernel_tma): each
-// work item's copies use its instance's tensor maps (b.tmaps_q, b.tmaps_fi); the tile
-// re-arms its two mbarriers per item.
-template <int FK, int LIM>
-__global__ void __launch_bounds__(256, (BatchResidency<float, 256>::value))
-    batch_stage_kernel_tma(const BatchArgs<float> b) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + StageSmemTma<8, 32>::bytes);
-  __shared__ StageArgs<float> sa;
-  __shared__ int item[3];  // instance, tile row, tile column
-  for (int w = blockIdx.x; w < b.nwork; w += gridDim.x) {
-    __syncthreads();  // the previous work item may still read shared memory
-    if (threadIdx.x == 0) {
-      const int packed = b.order[w];
-      const int k = packed >> 16, t = packed & 0xffff;
-      const int tj = b.inst[k].tiles_j;
-      sa = instance_args(b, k);
-      item[0] = k;
-      item[1] = t / tj;
-      item[2] = t % tj;
-    }
-    __syncthreads();
-    const int k = item[0];
-    stage_tile<8, 32, float, FK, float, false, false, 256, LIM, true>(sa, item[1], item[2], smem_raw,
-                                                                      b.tmaps_q + k, b.tmaps_fi + k, bars);
   }
 }
 

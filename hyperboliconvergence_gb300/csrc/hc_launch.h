@@ -4,7 +4,7 @@
 #pragma once
 
 #include "hc_kernels.cuh"
-#include "hc_tma.h"
+#include "hc_stage_warp.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -18,6 +18,16 @@ namespace hc {
 // TILE_AUTO (FP64 single-mesh default): 16x16_H, 8x8 or 4x8 by the mesh's size (f64_auto_tile)
 enum TileShape { TILE_8x32 = 0, TILE_4x32 = 1, TILE_16x16 = 2, TILE_16x16_H = 3, TILE_COUNT = 4, TILE_AUTO = 5,
                  TILE_8x8 = 6, TILE_4x8 = 7 };
+
+inline int device_sms() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 152;
+  }();
+  return sms;
+}
 
 // Tile of an FP64 stage launch.  The stage takes as long as its busiest SM, whose time is the
 // FP64 instructions of its tiles: an SM starts one per 19 cycles and each of its four
@@ -37,12 +47,7 @@ inline double f64_tile_cost(int ni, int nj, int ti, int tj, int sms) {
   return pass((ti + 1) * tj + ti * (tj + 1), 230) + pass((ti + 2) * (tj + 2), 48) + pass(ti * tj, 60);
 }
 inline int f64_auto_tile(int ni, int nj) {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 152;
-  }();
+  const int sms = device_sms();
   const double c16 = f64_tile_cost(ni, nj, 16, 16, sms), c8 = f64_tile_cost(ni, nj, 8, 8, sms),
                c4 = f64_tile_cost(ni, nj, 4, 8, sms);
   if (c16 <= c8 && c16 <= c4) return TILE_16x16_H;
@@ -80,6 +85,16 @@ template <class R>
 cudaError_t launch_scalar_batch_update0(const BatchArgs<R>& b, int tile, int grid, double cfl, R alpha00, R beta0,
                                         cudaStream_t s);
 
+// the strip kernel's arguments of one mesh
+inline StripArgs strip_args(const StageArgs<float>& a) {
+  StripArgs p{};
+  p.a = a;
+  p.strips = strip_count(a.nj);
+  p.rows = strip_run_rows(1, [&](int) { return a.ni; }, [&](int) { return a.nj; }, device_sms());
+  p.runs = (a.ni + p.rows - 1) / p.rows;
+  return p;
+}
+
 inline void tile_dims(int tile, int* ti, int* tj) {
   switch (tile) {
     case TILE_4x32: *ti = 4; *tj = 32; break;
@@ -108,48 +123,57 @@ inline void tile_dims(int tile, int* ti, int* tj) {
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,                             \
                                 int(StageSmem<TI, TJ, R>::bytes));                                       \
   }                                                                                                      \
-  /* FP32 kernels with the limiter a compile-time constant (the FP32 stage is bound by */               \
-  /* instruction issue; the run-time selection costs ~9% of it): the 8x32 single-mesh  */               \
-  /* tile for the common limiters, and every batch tile for van Albada and NoLimit3     */               \
-  /* with the state and i-face record loads staged by TMA where the mesh rows allow it */              \
-  template <int LIM> static void go_lim(const StageArgs<float>& a, cudaStream_t s) {                     \
-    const dim3 grid((a.nj + 31) / 32, (a.ni + 7) / 8);                                                   \
-    CUtensorMap tq, tfi;                                                                                 \
-    if (!a.plain_loads && stage_tma_maps(a, &tq, &tfi)) {                                                \
-      stage_kernel_tma<8, 32, float, FK, LIM, 256>                                                       \
-          <<<grid, 256, StageSmemTma<8, 32, float>::bytes + 2 * sizeof(uint64_t), s>>>(a, tq, tfi);      \
-      return;                                                                                            \
-    }                                                                                                    \
-    stage_kernel<8, 32, float, FK, float, 256, LIM><<<grid, 256, StageSmem<8, 32, float>::bytes, s>>>(a); \
-  }                                                                                                      \
-  static bool go_fixed_lim(const StageArgs<float>& a, cudaStream_t s) {                                  \
-    switch (a.limiter) {                                                                                 \
-      case LIM_VANALBADA: go_lim<LIM_VANALBADA>(a, s); return true;                                      \
-      case LIM_VANLEER: go_lim<LIM_VANLEER>(a, s); return true;                                          \
-      case LIM_MINMOD: go_lim<LIM_MINMOD>(a, s); return true;                                            \
-      case LIM_NOLIMIT2: go_lim<LIM_NOLIMIT2>(a, s); return true;                                        \
-      case LIM_NOLIMIT3: go_lim<LIM_NOLIMIT3>(a, s); return true;                                        \
-      default: return false;                                                                             \
-    }                                                                                                    \
-  }                                                                                                      \
-  template <int LIM> static void gob_tma(const BatchArgs<float>& b, int grid, cudaStream_t s) {          \
-    constexpr size_t smem = StageSmemTma<8, 32>::bytes + 2 * sizeof(uint64_t);                           \
-    static int cap = 0;                                                                                  \
-    if (cap == 0) {                                                                                      \
-      int dev = 0, sms = 0, occ = 0;                                                                     \
-      cudaGetDevice(&dev);                                                                               \
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);                                 \
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_stage_kernel_tma<FK, LIM>, 256, smem);   \
-      cap = (sms > 0 && occ > 0) ? sms * occ : grid;                                                     \
-    }                                                                                                    \
-    batch_stage_kernel_tma<FK, LIM><<<std::min(grid, cap), 256, smem, s>>>(b);                           \
-  }                                                                                                      \
+  /* FP32, primitive basis, the common limiters: the strip kernel (hc_stage_warp.cuh), with the    */   \
+  /* limiter a compile-time constant */                                                                 \
+  template <int LIM> static cudaError_t prep_strip() {                                                  \
+    cudaError_t e = cudaFuncSetAttribute(strip_kernel<FK, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,\
+                                         int(kStripSmem));                                              \
+    if (e != cudaSuccess) return e;                                                                     \
+    return cudaFuncSetAttribute(batch_strip_kernel<FK, LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,\
+                                int(kStripSmem));                                                       \
+  }                                                                                                     \
+  static cudaError_t prep_strips() {                                                                    \
+    cudaError_t e = prep_strip<LIM_VANALBADA>();                                                        \
+    if (e == cudaSuccess) e = prep_strip<LIM_VANLEER>();                                                \
+    if (e == cudaSuccess) e = prep_strip<LIM_MINMOD>();                                                 \
+    if (e == cudaSuccess) e = prep_strip<LIM_NOLIMIT2>();                                               \
+    if (e == cudaSuccess) e = prep_strip<LIM_NOLIMIT3>();                                               \
+    return e;                                                                                           \
+  }                                                                                                     \
+  template <int LIM> static bool go_strip(const StageArgs<float>& a, cudaStream_t s) {                  \
+    const StripArgs p = strip_args(a);                                                                  \
+    const unsigned grid = unsigned((p.strips * p.runs + kStripWarps - 1) / kStripWarps);                \
+    strip_kernel<FK, LIM><<<grid, 32 * kStripWarps, kStripSmem, s>>>(p);                                \
+    return true;                                                                                        \
+  }                                                                                                     \
+  static bool go_strips(const StageArgs<float>& a, cudaStream_t s) {                                    \
+    if (!a.pk || a.basis != 0 || a.dual_src) return false;                                              \
+    switch (a.limiter) {                                                                                \
+      case LIM_VANALBADA: return go_strip<LIM_VANALBADA>(a, s);                                         \
+      case LIM_VANLEER: return go_strip<LIM_VANLEER>(a, s);                                             \
+      case LIM_MINMOD: return go_strip<LIM_MINMOD>(a, s);                                               \
+      case LIM_NOLIMIT2: return go_strip<LIM_NOLIMIT2>(a, s);                                           \
+      case LIM_NOLIMIT3: return go_strip<LIM_NOLIMIT3>(a, s);                                           \
+      default: return false;                                                                            \
+    }                                                                                                   \
+  }                                                                                                     \
+  template <int LIM> static bool gob_strip(const BatchArgs<float>& b, cudaStream_t s) {                 \
+    batch_strip_kernel<FK, LIM><<<unsigned(b.strip_grid), 32 * kStripWarps, kStripSmem, s>>>(b);        \
+    return true;                                                                                        \
+  }                                                                                                     \
+  static bool gob_strips(const BatchArgs<float>& b, cudaStream_t s) {                                   \
+    if (!b.pk || b.basis != 0) return false;                                                            \
+    switch (b.limiter) {                                                                                \
+      case LIM_VANALBADA: return gob_strip<LIM_VANALBADA>(b, s);                                        \
+      case LIM_VANLEER: return gob_strip<LIM_VANLEER>(b, s);                                            \
+      case LIM_MINMOD: return gob_strip<LIM_MINMOD>(b, s);                                              \
+      case LIM_NOLIMIT2: return gob_strip<LIM_NOLIMIT2>(b, s);                                          \
+      case LIM_NOLIMIT3: return gob_strip<LIM_NOLIMIT3>(b, s);                                          \
+      default: return false;                                                                            \
+    }                                                                                                   \
+  }                                                                                                     \
   template <class R, int TI, int TJ, int LIM = -1>                                                        \
   static void gob(const BatchArgs<R>& b, int grid, cudaStream_t s) {                                     \
-    /* the TMA-staged tile where the batch has tensor maps for this stage's input */                    \
-    if constexpr (std::is_same<R, float>::value && TI == 8 && TJ == 32) {                                \
-      if (b.tmaps_q && b.tmaps_fi) { gob_tma<LIM>(b, grid, s); return; }                                  \
-    }                                                                                                    \
     /* a persistent grid larger than what stays resident would run a second, partial wave */           \
     static int cap = 0;                                                                                  \
     if (cap == 0) {                                                                                      \
@@ -177,6 +201,7 @@ inline void tile_dims(int tile, int* ti, int* tj) {
   }                                                                                                      \
   template <> cudaError_t launch_batch_stage<float, FK>(const BatchArgs<float>& b, int tile, int grid,   \
                                                         cudaStream_t s) {                                \
+    if (tile == TILE_8x32 && gob_strips(b, s)) return cudaGetLastError();                                \
     if (b.limiter == LIM_VANALBADA) gob_tile<LIM_VANALBADA>(b, tile, grid, s);                           \
     else if (b.limiter == LIM_NOLIMIT3) gob_tile<LIM_NOLIMIT3>(b, tile, grid, s);                        \
     else gob_tile<-1>(b, tile, grid, s);                                                                 \
@@ -203,6 +228,7 @@ inline void tile_dims(int tile, int* ti, int* tj) {
     if (e == cudaSuccess) e = prep_one<float, 4, 32>();                                                  \
     if (e == cudaSuccess) e = prep_one<float, 16, 16>();                                                 \
     if (e == cudaSuccess) e = prep_half<float>();                                                        \
+    if (e == cudaSuccess) e = prep_strips();                                                             \
     return e;                                                                                            \
   }                                                                                                      \
   template <class R> static cudaError_t dispatch(const StageArgs<R>& a, int tile, cudaStream_t s) {     \
@@ -214,7 +240,7 @@ inline void tile_dims(int tile, int* ti, int* tj) {
       return cudaGetLastError();                                                                         \
     }                                                                                                    \
     if constexpr (std::is_same<R, float>::value) {                                                       \
-      if ((tile == TILE_8x32 || tile < 0 || tile >= TILE_COUNT) && go_fixed_lim(a, s)) return cudaGetLastError(); \
+      if ((tile == TILE_8x32 || tile < 0 || tile >= TILE_COUNT) && go_strips(a, s)) return cudaGetLastError(); \
     }                                                                                                    \
     if constexpr (std::is_same<R, double>::value) {                                                      \
       if (tile == TILE_AUTO) tile = f64_auto_tile(a.ni, a.nj);                                           \

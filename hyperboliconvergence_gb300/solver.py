@@ -143,13 +143,13 @@ class Solver:
         check(self.lib.hc_set_corrections(self.h, self.corrections))
 
     def set_staged_loads(self, on: bool = True) -> None:
-        """The FP32 stage's tile loads staged by TMA tensor copies (the default) or plain
+        """The FP32 stage's face records staged by bulk copies (the default) or plain
         per-thread loads (hc_set_staged_loads); bit-identical results."""
         check(self.lib.hc_set_staged_loads(self.h, 1 if on else 0))
 
     def inject_stalled_copy(self, on: bool = True) -> None:
-        """Test hook of the failure detection (hc_inject_stalled_copy): the TMA-staged FP32
-        stage kernel's copy barrier waits for bytes that never come, its bounded wait runs out
+        """Test hook of the failure detection (hc_inject_stalled_copy): the FP32 strip
+        kernel's copy barrier waits for bytes that never come, its bounded wait runs out
         and the step raises HC_ERR_TIMEOUT with the context still usable."""
         check(self.lib.hc_inject_stalled_copy(self.h, 1 if on else 0))
 
