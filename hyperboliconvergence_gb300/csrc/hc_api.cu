@@ -262,6 +262,38 @@ template <class R> int run_step_1d(hc_ctx* c) {
   return HC_OK;
 }
 
+// nsteps steps of a short line (hc_oned.cuh, line_run_kernel)
+template <class R> int run_line(hc_ctx* c, int nsteps) {
+  const RKTab tab = rk_table(c->cfg.rk);
+  const Stage1DArgs<R> b = args_1d<R>(c);
+  LineRunArgs<R> a{};
+  a.nc = c->ni;
+  a.P.gas = b.gas;
+  a.P.limiter = b.limiter;
+  a.P.bc[0] = b.bc[0]; a.P.bc[1] = b.bc[1];
+  a.rec = b.rec;
+  a.vol = b.vol;
+  a.gref[0] = b.gref[0]; a.gref[1] = b.gref[1];
+  a.q = (R*)c->q[0];
+  a.nst = tab.nst;
+  a.global = c->cfg.dt_mode == HC_DT_GLOBAL;
+  for (int s = 0; s < tab.nst; ++s) {
+    a.beta[s] = R(tab.beta[s]);
+    for (int k = 0; k <= s; ++k) a.alpha[s][k] = R(tab.alpha[s][k]);
+  }
+  a.cfl = b.cfl;
+  a.dcfl = c->cfg.cfl;
+  a.info = c->info;
+  while (nsteps > 0) {
+    a.nsteps = std::min(nsteps, kLineChunk);
+    nsteps -= a.nsteps;
+    HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
+    HC_CUDA(launch_line_run<R>(a, c->cfg.flux, c->stream));
+    c->launches += 1;
+  }
+  return HC_OK;
+}
+
 template <class R> int run_residual(hc_ctx* c) {
   if (c->oned) return run_residual_1d<R>(c);
   StageArgs<R> a = base_args<R>(c);
@@ -888,6 +920,8 @@ int hc_step_async(hc_ctx* c, int nsteps) {
   if (int st = ensure_ready(c)) return st;
   // clear the device status of earlier calls (status and bad_cell are adjacent ints)
   HC_CUDA(cudaMemsetAsync(&c->info->status, 0, 2 * sizeof(int), c->stream));
+  if (c->oned && c->ni <= kLineMax && !(c->smooth_alpha > 0.0))
+    return c->fp32 ? run_line<float>(c, nsteps) : run_line<double>(c, nsteps);
   for (int k = 0; k < nsteps; ++k) {
     const int st = c->fp32 ? run_step<float>(c) : run_step<double>(c);
     if (st != HC_OK) return st;
