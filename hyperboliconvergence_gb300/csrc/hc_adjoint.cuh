@@ -34,11 +34,6 @@ template <class R> __host__ __device__ __forceinline__ void prim_state_adj_ir(co
   qbar[2] += sb.r;
   qbar[3] += sb.p;
 }
-template <class R> __host__ __device__ __forceinline__ void prim_state_adj(const Gas<R>& g, const R* q, StBar<R>& sb,
-                                                                  R* qbar) {
-  prim_state_adj_ir(g, q, R(1) / q[2], sb, qbar);
-}
-
 // exact flux adjoint, accumulating into the state adjoint of one side
 template <class R> __host__ __device__ __forceinline__ void exact_flux_adj(R nx, R ny, const St<R>& s, const R* fbar,
                                                                   StBar<R>& sb) {
@@ -65,9 +60,11 @@ template <class R> __host__ __device__ __forceinline__ void entropy_fix_adj(R la
   R laabar, lebar = R(0);
   if (laa > le) {
     laabar = lbar;
-  } else {
+  } else if (le > R(0)) {
     lebar = R(0.5) * (R(1) - laa * laa / (le * le)) * lbar;
     laabar = (laa / le) * lbar;
+  } else {
+    laabar = R(0);  // exactly sonic, no expansion: the speed is 0 (roe_flux)
   }
   *labar += sgn(la) * laabar;
   if (mx > R(0)) {
@@ -77,170 +74,157 @@ template <class R> __host__ __device__ __forceinline__ void entropy_fix_adj(R la
   }
 }
 
-// Reverse of roe_flux (hc_physics.cuh) for the four conserved flux components,
-// with respect to the two primitive face states.
+// v with the sign of s, 0 where s is 0: v sgn(s) without an FP64 comparison
+template <class R> __host__ __device__ __forceinline__ R times_sgn(R v, R s) { return sgn(s) * v; }
+template <> __host__ __device__ __forceinline__ double times_sgn<double>(double v, double s) {
+  const long long b = f64_bits(s);
+  return (b << 1) == 0 ? 0.0 : (b < 0 ? -v : v);
+}
+
+// Reverse of roe_flux (hc_physics.cuh) for the four conserved flux components, with respect to
+// the two primitive face states.  It reverses the multiplied-out form of the flux, in which the
+// averaged density appears only through the averaging weight, and takes the sound speeds of the
+// two states only where Harten's fix may act: 230 FP64 instructions with the forward values,
+// against 330 for the transforms one by one.
 template <class R>
 __host__ __device__ __forceinline__ void roe_flux_adj(const Gas<R>& g, R nx, R ny, R A, const R* ql, const R* qr,
                                              const R* Fbar, R* qlbar, R* qrbar) {
-  // FP64: the two inverse densities from one division, the sound speeds and their
-  // inverses from reciprocal square roots (as the forward stage computes them)
   St<R> l, r;
   basis_state2(g, ql, qr, false, l, r);
-  // ---- forward recomputation (reciprocals: l.ir = 1/rL, r.ir = 1/rR, a1 = 1/aa)
-  const R z = r.r * l.ir;
-  const R cr = sqrt(z);
-  const R icr = cr * l.r * r.ir;  // 1/cr
-  const R wl = R(1) / (R(1) + cr);
+  // ---- forward values
+  const R unl = proj(nx, ny, l), unr = proj(nx, ny, r);
+  R cr;
+  sqrt_fast(r.r * l.ir, cr);
+  const R wl = rcp_fast(R(1) + cr);
   const R wr = R(1) - wl;
-  const R ra = cr * l.r;
-  const R ua = wl * l.u + wr * r.u;
-  const R va = wl * l.v + wr * r.v;
-  const R ka = R(0.5) * (ua * ua + va * va);
-  const R ha = wl * l.h + wr * r.h;
-  const R a2a = g.gm1 * (ha - ka);
-  R aa, a1, al, ial, ar, iar;
-  sqrt_rcp(a2a, aa, a1);
-  sqrt_rcp(l.a2, al, ial);
-  sqrt_rcp(r.a2, ar, iar);
-  const R una = nx * ua + ny * va;
-  const R unl = nx * l.u + ny * l.v, unr = nx * r.u + ny * r.v;
-  const R la1 = una - aa, ll1 = unl - al, lr1 = unr - ar;
-  const R la2 = una + aa, ll2 = unl + al, lr2 = unr + ar;
-  auto fix = [](R la, R ll, R lr) {
-    const R le = R(0.05) * fmax(R(0), fmax(la - ll, lr - la));
-    const R laa = fabs(la);
-    return (laa > le) ? laa : R(0.5) * (le + laa * laa / le);
-  };
-  const R lam0 = fabs(una), lam1 = fix(la1, ll1, lr1), lam2 = fix(la2, ll2, lr2), lam3 = lam0;
-  const R tx = -ny, ty = nx;
-  const R d0 = r.r * r.u - l.r * l.u;
-  const R d1 = r.r * r.v - l.r * l.v;
+  const R ua = mad(wl, l.u, wr * r.u);
+  const R va = mad(wl, l.v, wr * r.v);
+  const R ka = R(0.5) * mad(va, va, ua * ua);
+  const R ha = mad(wl, l.h, wr * r.h);
+  R aa, a1;
+  sqrt_rcp(g.gm1 * (ha - ka), aa, a1);
+  const R una = mad(nx, ua, ny * va);
+  const R la1 = una - aa, la2 = una + aa;
+  const R lam0 = fabs(una);
+  R h1 = R(0.5) * fabs(la1), h2 = R(0.5) * fabs(la2);
+  const bool near_fix = harten_near(unl, unr, l.a2, r.a2, una, aa);
+  R al = R(0), ar = R(0), ial = R(0), iar = R(0);
+  if (near_fix) {
+    sqrt_rcp(l.a2, al, ial);
+    sqrt_rcp(r.a2, ar, iar);
+    auto fix = [](R la, R ll, R lr, R h) {
+      const R le = R(0.05) * fmax(R(0), fmax(la - ll, lr - la));
+      const R laa = fabs(la);
+      return (laa > le || !(le > R(0))) ? h : R(0.25) * (le + laa * laa / le);
+    };
+    h1 = fix(la1, unl - al, unr - ar, h1);
+    h2 = fix(la2, unl + al, unr + ar, h2);
+  }
+  const R d0 = mad(r.r, r.u, -(l.r * l.u));
+  const R d1 = mad(r.r, r.v, -(l.r * l.v));
   const R d2 = r.r - l.r;
-  const R d3 = (r.r * r.h - r.p) - (l.r * l.h - l.p);
-  const R c0 = nx * d0 + ny * d1;
-  const R c1 = tx * d0 + ty * d1;
-  const R rho1 = cr * r.ir;  // 1/ra
-  const R cc = ka * d2 + d3 - ua * c0 - va * c1;
-  const R du0 = (c0 - ua * d2) * rho1;
-  const R du1 = (c1 - va * d2) * rho1;
-  const R dp = cc * g.gm1;
-  const R X0 = g.gamma * (dp * a1 * a1 - d2) * rho1;
-  const R X1 = du0 - dp * rho1 * a1;
-  const R X2 = du0 + dp * rho1 * a1;
-  const R w0 = lam0 * X0, w1 = lam1 * X1, w2 = lam2 * X2, w3 = lam3 * du1;
-  const R dpp = R(0.5) * ra * aa * (w2 - w1);
-  const R drr = dpp * (a1 * a1) - ra * w0 * g.inv_gamma;
-  const R du = R(0.5) * (w1 + w2);
-  const R dv = w3;
-  const R dk = ua * du + va * dv;
-  // ---- reverse
-  const R s = R(-0.5) * A;
-  const R f0b = s * Fbar[0], f1b = s * Fbar[1];
-  R drrb = s * Fbar[2];
-  const R e3b = s * Fbar[3];
-  const R e0b = nx * f0b + ny * f1b;
-  const R e1b = tx * f0b + ty * f1b;
-  R dppb = g.gamma1 * e3b;
-  R rab = dk * e3b;
-  const R dkb = ra * e3b;
+  const R d3 = mad(r.r, r.h, -r.p) - mad(l.r, l.h, -l.p);
+  const R c0 = mad(nx, d0, ny * d1);
+  const R c1 = mad(nx, d1, -(ny * d0));
+  const R dp = g.gm1 * mad(-va, c1, mad(-ua, c0, mad(ka, d2, d3)));
+  const R cn = mad(-ua, d2, c0), da = dp * a1;
+  const R m1 = cn - da, m2 = cn + da;
+  const R w1 = h1 * m1, w2 = h2 * m2;
+  const R a12 = a1 * a1;
+  const R z = mad(dp, a12, -d2);
+  const R sm = w1 + w2, df = w2 - w1;
+  const R drr = mad(-lam0, z, df * a1);
+  const R t = mad(-va, d2, c1);
+  const R sh = lam0 * t;
+  // ---- reverse: G the adjoint of the central sums, -G of the dissipation's
+  const R hA = R(0.5) * A;
+  const R G0 = hA * Fbar[0], G1 = hA * Fbar[1], G2 = hA * Fbar[2], G3 = hA * Fbar[3];
+  const R pn = mad(nx, G0, ny * G1);
+  const R e0b = -pn, e1b = mad(ny, G0, -(nx * G1)), e3b = -G3;
+  const R dppb = g.gamma1 * e3b;
+  const R smb = mad(ua, e3b, e0b);
+  const R shb = mad(va, e3b, e1b);
+  const R drrb = mad(ua, e0b, mad(va, e1b, mad(ka, e3b, -G2)));
+  R uab = mad(drr, e0b, sm * e3b);
+  R vab = mad(drr, e1b, sh * e3b);
   R kab = drr * e3b;
-  drrb += ka * e3b;
-  R uab = du * dkb, vab = dv * dkb;
-  R dub = ua * dkb, dvb = va * dkb;
-  rab += dv * e1b; dvb += ra * e1b; vab += drr * e1b; drrb += va * e1b;
-  rab += du * e0b; dub += ra * e0b; uab += drr * e0b; drrb += ua * e0b;
-  R w3b = dvb;
-  R w1b = R(0.5) * dub, w2b = R(0.5) * dub;
-  dppb += drrb * (a1 * a1);
-  R aab = R(-2) * dpp * (a1 * a1 * a1) * drrb;
-  rab += -w0 * g.inv_gamma * drrb;
-  R w0b = -ra * g.inv_gamma * drrb;
-  rab += R(0.5) * aa * (w2 - w1) * dppb;
-  aab += R(0.5) * ra * (w2 - w1) * dppb;
-  w2b += R(0.5) * ra * aa * dppb;
-  w1b -= R(0.5) * ra * aa * dppb;
-  R lam0b = X0 * w0b, lam1b = X1 * w1b, lam2b = X2 * w2b, lam3b = du1 * w3b;
-  const R X0b = lam0 * w0b, X1b = lam1 * w1b, X2b = lam2 * w2b;
-  R du1b = lam3 * w3b;
-  R du0b = X1b + X2b;
-  R dpb = rho1 * a1 * (X2b - X1b);
-  R rho1b = dp * a1 * (X2b - X1b);
-  R a1b = dp * rho1 * (X2b - X1b);
-  dpb += g.gamma * a1 * a1 * rho1 * X0b;
-  a1b += g.gamma * R(2) * dp * a1 * rho1 * X0b;
-  R d2b = -g.gamma * rho1 * X0b;
-  rho1b += g.gamma * (dp * a1 * a1 - d2) * X0b;
-  aab += -a1 * a1 * a1b;
-  const R ccb = g.gm1 * dpb;
-  R c1b = rho1 * du1b;
-  vab -= d2 * rho1 * du1b;
-  d2b -= va * rho1 * du1b;
-  rho1b += (c1 - va * d2) * du1b;
-  R c0b = rho1 * du0b;
-  uab -= d2 * rho1 * du0b;
-  d2b -= ua * rho1 * du0b;
-  rho1b += (c0 - ua * d2) * du0b;
-  kab += d2 * ccb; d2b += ka * ccb;
-  const R d3b = ccb;
-  uab -= c0 * ccb; c0b -= ua * ccb;
-  vab -= c1 * ccb; c1b -= va * ccb;
-  rab += -rho1 * rho1 * rho1b;
-  const R d0b = nx * c0b + tx * c1b;
-  const R d1b = ny * c0b + ty * c1b;
-  StBar<R> lb{}, rb{};
-  rb.r += r.u * d0b; rb.u += r.r * d0b; lb.r -= l.u * d0b; lb.u -= l.r * d0b;
-  rb.r += r.v * d1b; rb.v += r.r * d1b; lb.r -= l.v * d1b; lb.v -= l.r * d1b;
-  rb.r += d2b; lb.r -= d2b;
-  rb.r += r.h * d3b; rb.h += r.r * d3b; rb.p -= d3b;
-  lb.r -= l.h * d3b; lb.h -= l.r * d3b; lb.p += d3b;
+  // the waves
+  const R lam0b = mad(t, shb, -(z * drrb));
+  const R tb = lam0 * shb, zb = -(lam0 * drrb);
+  const R dfb = mad(a1, drrb, aa * dppb);
+  R aab = df * dppb;
+  R a1b = df * drrb;
+  const R w1b = smb - dfb, w2b = smb + dfb;
+  const R m1b = h1 * w1b, m2b = h2 * w2b;
+  const R lam1b = R(0.5) * (m1 * w1b), lam2b = R(0.5) * (m2 * w2b);
+  const R cnb = m1b + m2b, dab = m2b - m1b;
+  const R dpb = mad(a12, zb, a1 * dab);
+  a1b = mad(R(2) * da, zb, mad(dp, dab, a1b));
+  // the pressure jump and the jumps in the face frame
+  const R q = g.gm1 * dpb;
+  kab = mad(d2, q, kab);
+  uab = mad(-d2, cnb, mad(-c0, q, uab));
+  vab = mad(-d2, tb, mad(-c1, q, vab));
+  const R c0b = mad(-ua, q, cnb), c1b = mad(-va, q, tb);
+  const R d2b = mad(ka, q, mad(-ua, cnb, mad(-va, tb, -zb)));
+  const R d0b = mad(nx, c0b, -(ny * c1b));
+  const R d1b = mad(ny, c0b, nx * c1b);
   // wave speeds
-  R unab = sgn(una) * (lam0b + lam3b);
-  R la1b = R(0), ll1b = R(0), lr1b = R(0), la2b = R(0), ll2b = R(0), lr2b = R(0);
-  entropy_fix_adj(la1, ll1, lr1, lam1b, &la1b, &ll1b, &lr1b);
-  entropy_fix_adj(la2, ll2, lr2, lam2b, &la2b, &ll2b, &lr2b);
-  unab += la1b + la2b;
-  aab += la2b - la1b;
-  const R unlb = ll1b + ll2b, unrb = lr1b + lr2b;
-  const R alb = ll2b - ll1b, arb = lr2b - lr1b;
-  lb.a2 += alb * (R(0.5) * ial);
-  rb.a2 += arb * (R(0.5) * iar);
-  lb.u += nx * unlb; lb.v += ny * unlb;
-  rb.u += nx * unrb; rb.v += ny * unrb;
-  uab += nx * unab; vab += ny * unab;
-  const R a2ab = aab * (R(0.5) * a1);
-  const R hab = g.gm1 * a2ab;
-  kab -= g.gm1 * a2ab;
-  uab += ua * kab; vab += va * kab;
-  R wlb = l.h * hab + l.u * uab + l.v * vab;
-  const R wrb = r.h * hab + r.u * uab + r.v * vab;
-  lb.h += wl * hab; rb.h += wr * hab;
-  lb.u += wl * uab; rb.u += wr * uab;
-  lb.v += wl * vab; rb.v += wr * vab;
-  R crb = l.r * rab;
-  lb.r += cr * rab;
-  wlb -= wrb;
-  crb += -wl * wl * wlb;
-  const R zb = crb * (R(0.5) * icr);
-  rb.r += zb * l.ir;
-  lb.r -= zb * z * l.ir;
-  // central part: c.f[i] = 0.5*(fl[i]+fr[i])*A
-  R fe[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) fe[i] = R(0.5) * A * Fbar[i];
-  exact_flux_adj(nx, ny, l, fe, lb);
-  exact_flux_adj(nx, ny, r, fe, rb);
-  prim_state_adj_ir(g, ql, l.ir, lb, qlbar);
-  prim_state_adj_ir(g, qr, r.ir, rb, qrbar);
+  R unab, unlb = R(0), unrb = R(0), la2l = R(0), la2r = R(0);
+  {
+    R la1b = R(0), la2b = R(0);
+    if (near_fix) {
+      R ll1b = R(0), lr1b = R(0), ll2b = R(0), lr2b = R(0);
+      entropy_fix_adj(la1, unl - al, unr - ar, lam1b, &la1b, &ll1b, &lr1b);
+      entropy_fix_adj(la2, unl + al, unr + ar, lam2b, &la2b, &ll2b, &lr2b);
+      unlb = ll1b + ll2b;
+      unrb = lr1b + lr2b;
+      la2l = (ll2b - ll1b) * (R(0.5) * ial);
+      la2r = (lr2b - lr1b) * (R(0.5) * iar);
+    } else {
+      la1b = times_sgn(lam1b, la1);
+      la2b = times_sgn(lam2b, la2);
+    }
+    unab = times_sgn(lam0b, una) + (la1b + la2b);
+    aab = mad(-a12, a1b, aab) + (la2b - la1b);
+  }
+  uab = mad(nx, unab, uab);
+  vab = mad(ny, unab, vab);
+  const R hab = (R(0.5) * g.gm1) * (a1 * aab);
+  kab = kab - hab;
+  uab = mad(ua, kab, uab);
+  vab = mad(va, kab, vab);
+  // the averaging weight
+  const R wlb = mad(l.h - r.h, hab, mad(l.u - r.u, uab, (l.v - r.v) * vab));
+  const R k = (R(-0.5) * cr) * ((wl * wl) * wlb);
+  // the two states: jumps, averages and central fluxes
+  auto side = [&](const St<R>& s, const R* qs, R un, R w, R sg, R unb, R a2x, R* qbar) {
+    const R mnb = mad(s.u, G0, mad(s.v, G1, mad(s.h, G3, G2)));
+    const R ub = mad(s.r, mad(nx, mnb, mad(un, G0, sg * d0b)), mad(nx, unb, w * uab));
+    const R vb = mad(s.r, mad(ny, mnb, mad(un, G1, sg * d1b)), mad(ny, unb, w * vab));
+    const R hb = mad(s.r, mad(un, G3, sg * q), w * hab);
+    const R rb = mad(un, mnb, sg * mad(s.u, d0b, mad(s.v, d1b, mad(s.h, q, mad(k, s.ir, d2b)))));
+    // primitive -> state (prim_state_adj)
+    const R gb = (g.gamma * s.ir) * mad(g.gamma1, hb, a2x);
+    qbar[0] += mad(qs[0], hb, ub);
+    qbar[1] += mad(qs[1], hb, vb);
+    qbar[2] += mad(-gb, qs[3] * s.ir, rb);
+    qbar[3] += gb + mad(-sg, q, pn);
+  };
+  side(l, ql, unl, wl, R(-1), unlb, la2l, qlbar);
+  side(r, qr, unr, wr, R(1), unrb, la2r, qrbar);
 }
 
 // Reverse of rusanov_flux (conservationLaws/base/fluxes/rusanovFlux.ipp:2-50)
 template <class R>
 __host__ __device__ __forceinline__ void rusanov_flux_adj(const Gas<R>& g, R nx, R ny, R A, const R* ql, const R* qr,
                                                  const R* Fbar, R* qlbar, R* qrbar) {
-  const St<R> l = prim_state(g, ql[0], ql[1], ql[2], ql[3]);
-  const St<R> r = prim_state(g, qr[0], qr[1], qr[2], qr[3]);
-  const R unl = nx * l.u + ny * l.v, unr = nx * r.u + ny * r.v;
-  const R al = sqrt(l.a2), ar = sqrt(r.a2);
+  St<R> l, r;
+  basis_state2(g, ql, qr, false, l, r);
+  const R unl = proj(nx, ny, l), unr = proj(nx, ny, r);
+  R al, ar;
+  sqrt_fast(l.a2, al);
+  sqrt_fast(r.a2, ar);
   const R srl = fabs(unl) + al, srr = fabs(unr) + ar;
   const R lambda = fmax(srl, srr);
   const R s = R(-0.5) * (lambda * A);
@@ -257,67 +241,46 @@ __host__ __device__ __forceinline__ void rusanov_flux_adj(const Gas<R>& g, R nx,
   rb.r += r.h * s * Fbar[3]; rb.h += r.r * s * Fbar[3]; rb.p -= s * Fbar[3];
   lb.r -= l.h * s * Fbar[3]; lb.h -= l.r * s * Fbar[3]; lb.p += s * Fbar[3];
   if (srl >= srr) {
-    lb.u += nx * sgn(unl) * lamb; lb.v += ny * sgn(unl) * lamb; lb.a2 += lamb / (R(2) * al);
+    lb.u += nx * sgn(unl) * lamb; lb.v += ny * sgn(unl) * lamb; lb.a2 += div_fast(lamb, R(2) * al);
   } else {
-    rb.u += nx * sgn(unr) * lamb; rb.v += ny * sgn(unr) * lamb; rb.a2 += lamb / (R(2) * ar);
+    rb.u += nx * sgn(unr) * lamb; rb.v += ny * sgn(unr) * lamb; rb.a2 += div_fast(lamb, R(2) * ar);
   }
   R fe[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) fe[i] = R(0.5) * A * Fbar[i];
   exact_flux_adj(nx, ny, l, fe, lb);
   exact_flux_adj(nx, ny, r, fe, rb);
-  prim_state_adj(g, ql, lb, qlbar);
-  prim_state_adj(g, qr, rb, qrbar);
+  prim_state_adj_ir(g, ql, l.ir, lb, qlbar);
+  prim_state_adj_ir(g, qr, r.ir, rb, qrbar);
 }
 
 // van Albada's value z = ab(a+b)/(a^2+b^2+tiny) and its derivatives along the taken branch
-// for four (a, b) pairs, FP64: 0 with zero derivatives where a b < 0 or a = b = 0 (the
-// formula's own derivatives there); otherwise the four inverse denominators from one
-// division (batched inversion) when every denominator lies in [2^-240, 2^240], one
-// division each when not.  The sign and range tests read the bits on the integer pipe.
+// for four (a, b) pairs, FP64, 17 instructions each: 0 with zero derivatives where a b < 0 or
+// a = b = 0 (the formula's own derivatives there).  The sign and range tests read the bits on
+// the integer pipe.
 __host__ __device__ __forceinline__ void vanalbada_vg4(const double* a, const double* b, double* z, double* da,
                                                        double* db) {
-  double den[4], pre[4], iden[4];
-  double acc = 1.0;
-  bool ok = true, any = false;
-  bool on[4];
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
-    const long long bits = f64_bits(a[v] * b[v]);
+    const double ab = a[v] * b[v];
+    const long long bits = f64_bits(ab);
     const unsigned long long mag = (unsigned long long)bits << 1;  // magnitude bits
     // not (a b < 0): a b is +0, -0, positive or NaN (which propagates); and not a = b = 0
     const bool both_zero = ((unsigned long long)f64_bits(a[v]) << 1) == 0 && ((unsigned long long)f64_bits(b[v]) << 1) == 0;
-    on[v] = (bits >= 0 || mag == 0 || mag > (0x7ff0000000000000ULL << 1)) && !both_zero;
-    den[v] = on[v] ? fma(a[v], a[v], b[v] * b[v]) : 1.0;
-    any = any || on[v];
-    pre[v] = acc;
-    acc = acc * den[v];
-    ok = ok && f64_exp_within(den[v], 240u);
-  }
-  if (!any) {
-#pragma unroll
-    for (int v = 0; v < 4; ++v) z[v] = da[v] = db[v] = 0.0;
-    return;
-  }
-  if (ok) {
-    double inv = 1.0 / acc;
-#pragma unroll
-    for (int v = 3; v >= 0; --v) {
-      iden[v] = inv * pre[v];
-      inv = inv * den[v];
-    }
-  } else {
-#pragma unroll
-    for (int v = 0; v < 4; ++v) iden[v] = 1.0 / (den[v] + Lim<double>::tiny());
-  }
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    if (!on[v]) { z[v] = da[v] = db[v] = 0.0; continue; }
-    const double a2 = a[v] * a[v], b2 = b[v] * b[v], ab2 = 2.0 * a[v] * b[v];
-    const double zz = (b[v] * a2 + a[v] * b2) * iden[v];
+    const bool on = (bits >= 0 || mag == 0 || mag > (0x7ff0000000000000ULL << 1)) && !both_zero;
+    if (!on) { z[v] = da[v] = db[v] = 0.0; continue; }
+    const double a2 = a[v] * a[v], b2 = b[v] * b[v], den = a2 + b2;
+    double iden;
+#ifdef __CUDA_ARCH__
+    if (f64_in_window(den)) iden = rcp_step(den);
+    else
+#endif
+      iden = 1.0 / (den + Lim<double>::tiny());
+    const double ab2 = ab + ab;
+    const double zz = (ab * (a[v] + b[v])) * iden;
     z[v] = zz;
-    da[v] = ((ab2 + b2) - zz * 2.0 * a[v]) * iden[v];
-    db[v] = ((a2 + ab2) - zz * 2.0 * b[v]) * iden[v];
+    da[v] = fma(-zz, a[v] + a[v], ab2 + b2) * iden;
+    db[v] = fma(-zz, b[v] + b[v], a2 + ab2) * iden;
   }
 }
 
@@ -333,7 +296,7 @@ template <class R> __host__ __device__ __forceinline__ void limit_grad(int kind,
       if (a * b < R(0)) return;
       // z = num/den; dz = (dnum - z*dden)/den (no den^2: it underflows at a = b = 0)
       const R num = b * (a * a) + a * (b * b), den = a * a + b * b + tiny;
-      const R iden = R(1) / den;
+      const R iden = rcp_fast(den);
       const R z = num * iden;
       *da = ((R(2) * a * b + b * b) - z * R(2) * a) * iden;
       *db = ((a * a + R(2) * a * b) - z * R(2) * b) * iden;
@@ -345,7 +308,7 @@ template <class R> __host__ __device__ __forceinline__ void limit_grad(int kind,
       return;
     case LIM_VANLEER: {
       const R num = a * fabs(b) + fabs(a) * b, den = fabs(a) + fabs(b) + tiny;
-      const R iden = R(1) / den;
+      const R iden = rcp_fast(den);
       const R z = num * iden;
       *da = ((fabs(b) + sgn(a) * b) - z * sgn(a)) * iden;
       *db = ((a * sgn(b) + fabs(a)) - z * sgn(b)) * iden;
@@ -361,7 +324,7 @@ template <class R> __host__ __device__ __forceinline__ void limit_grad(int kind,
 // (one reciprocal of the density and the gas's 1/(gamma-1) instead of four divisions: the
 // reverse passes are bound by the FP64 pipe)
 template <class R> __host__ __device__ __forceinline__ void cons2prim_adj(const Gas<R>& g, const R* q, const R* pb, R* cb) {
-  const R u = q[0], v = q[1], ir = R(1) / q[2];
+  const R u = q[0], v = q[1], ir = rcp_fast(q[2]);
   cb[0] = pb[0] * ir - g.gm1 * u * pb[3];
   cb[1] = pb[1] * ir - g.gm1 * v * pb[3];
   cb[2] = pb[2] - (u * pb[0] + v * pb[1]) * ir + R(0.5) * g.gm1 * (u * u + v * v) * pb[3];

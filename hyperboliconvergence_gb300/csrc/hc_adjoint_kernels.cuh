@@ -157,8 +157,9 @@ __device__ __forceinline__ void adj_face_one(const AdjArgs<R>& a, int dir, int f
         for (int v = 0; v < 4; ++v) {
           const C dq = qr[v] - ql[v];
           gc[v] = dq * idlr;
-          gl[v] = (a.qm[(2 * v) * n + cl] * wlx + a.qm[(2 * v + 1) * n + cl] * wly) - dq * sl;
-          gr[v] = (a.qm[(2 * v) * n + cr] * wrx + a.qm[(2 * v + 1) * n + cr] * wry) - dq * sr;
+          // (contracted as the forward stage does)
+          gl[v] = mad(-dq, sl, mad(C(a.qm[(2 * v + 1) * n + cl]), wly, C(a.qm[(2 * v) * n + cl]) * wlx));
+          gr[v] = mad(-dq, sr, mad(C(a.qm[(2 * v + 1) * n + cr]), wry, C(a.qm[(2 * v) * n + cr]) * wrx));
         }
         if constexpr (f64) {
           if (vg) {
@@ -167,8 +168,8 @@ __device__ __forceinline__ void adj_face_one(const AdjArgs<R>& a, int dir, int f
             vanalbada_vg4(gc, gr, zr, dar, dbr);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-              qL[v] = ql[v] + dl * zl[v];
-              qR[v] = qr[v] - dr * zr[v];
+              qL[v] = mad(dl, C(zl[v]), ql[v]);
+              qR[v] = mad(-dr, C(zr[v]), qr[v]);
             }
           }
         }
@@ -187,14 +188,14 @@ __device__ __forceinline__ void adj_face_one(const AdjArgs<R>& a, int dir, int f
           if (vg) { da = dal[v]; db = dbl[v]; }
           else limit_grad<C>(lim, gc[v], gl[v], &da, &db);
           const C zlb = dl * qLb[v];
-          C gcb = zlb * da;
+          const C gcl = zlb * da;
           const C glb = zlb * db;
           if (vg) { da = dar[v]; db = dbr[v]; }
           else limit_grad<C>(lim, gc[v], gr[v], &da, &db);
           const C zrb = -dr * qRb[v];
-          gcb += zrb * da;
+          const C gcb = mad(zrb, da, gcl);
           const C grb = zrb * db;
-          const C dqb = gcb * idlr - glb * sl - grb * sr;
+          const C dqb = mad(-grb, sr, mad(-glb, sl, gcb * idlr));
           dL[v] = qLb[v] - dqb;
           dR[v] = qRb[v] + dqb;
           gL[v] = glb;
@@ -497,7 +498,7 @@ __device__ __forceinline__ void adj_update_lin_cell(int ncell, const R* __restri
                                                     R alpha3, int stage, R dts, int c) {
   if (c >= ncell) return;
   const size_t n = size_t(ncell);
-  const R fac = dts / vol[c];
+  const R fac = div_fast(dts, vol[c]);
   R* rb[4] = {rbar0, rbar1, rbar2, rbar3};
   const R al[4] = {alpha0, alpha1, alpha2, alpha3};
 #pragma unroll
@@ -617,7 +618,7 @@ __device__ __forceinline__ void adj_update_apply(const Gas<R>& g, const R* __res
   for (int v = 0; v < 4; ++v) { q[v] = q_out[v * n + c]; qz[v] = q0[v * n + c]; }
   cons2prim_adj(g, q, qb, cb);
   prim2cons_adj(g, qz, cb, z);
-  const R fac = dts / vol[c];
+  const R fac = div_fast(dts, vol[c]);
   if (first) {
 #pragma unroll
     for (int v = 0; v < 4; ++v) q0bar[v * n + c] = z[v];
