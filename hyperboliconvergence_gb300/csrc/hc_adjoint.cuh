@@ -296,7 +296,7 @@ template <class R> __host__ __device__ __forceinline__ void limit_grad(int kind,
       if (a * b < R(0)) return;
       // z = num/den; dz = (dnum - z*dden)/den (no den^2: it underflows at a = b = 0)
       const R num = b * (a * a) + a * (b * b), den = a * a + b * b + tiny;
-      const R iden = rcp_fast(den);
+      const R iden = rcp_near(den);
       const R z = num * iden;
       *da = ((R(2) * a * b + b * b) - z * R(2) * a) * iden;
       *db = ((a * a + R(2) * a * b) - z * R(2) * b) * iden;
@@ -308,7 +308,7 @@ template <class R> __host__ __device__ __forceinline__ void limit_grad(int kind,
       return;
     case LIM_VANLEER: {
       const R num = a * fabs(b) + fabs(a) * b, den = fabs(a) + fabs(b) + tiny;
-      const R iden = rcp_fast(den);
+      const R iden = rcp_near(den);
       const R z = num * iden;
       *da = ((fabs(b) + sgn(a) * b) - z * sgn(a)) * iden;
       *db = ((a * sgn(b) + fabs(a)) - z * sgn(b)) * iden;
@@ -324,7 +324,7 @@ template <class R> __host__ __device__ __forceinline__ void limit_grad(int kind,
 // (one reciprocal of the density and the gas's 1/(gamma-1) instead of four divisions: the
 // reverse passes are bound by the FP64 pipe)
 template <class R> __host__ __device__ __forceinline__ void cons2prim_adj(const Gas<R>& g, const R* q, const R* pb, R* cb) {
-  const R u = q[0], v = q[1], ir = rcp_fast(q[2]);
+  const R u = q[0], v = q[1], ir = rcp_near(q[2]);
   cb[0] = pb[0] * ir - g.gm1 * u * pb[3];
   cb[1] = pb[1] * ir - g.gm1 * v * pb[3];
   cb[2] = pb[2] - (u * pb[0] + v * pb[1]) * ir + R(0.5) * g.gm1 * (u * u + v * v) * pb[3];

@@ -498,7 +498,7 @@ __device__ __forceinline__ void adj_update_lin_cell(int ncell, const R* __restri
                                                     R alpha3, int stage, R dts, int c) {
   if (c >= ncell) return;
   const size_t n = size_t(ncell);
-  const R fac = div_fast(dts, vol[c]);
+  const R fac = div_near(dts, vol[c]);
   R* rb[4] = {rbar0, rbar1, rbar2, rbar3};
   const R al[4] = {alpha0, alpha1, alpha2, alpha3};
 #pragma unroll
@@ -618,7 +618,7 @@ __device__ __forceinline__ void adj_update_apply(const Gas<R>& g, const R* __res
   for (int v = 0; v < 4; ++v) { q[v] = q_out[v * n + c]; qz[v] = q0[v * n + c]; }
   cons2prim_adj(g, q, qb, cb);
   prim2cons_adj(g, qz, cb, z);
-  const R fac = div_fast(dts, vol[c]);
+  const R fac = div_near(dts, vol[c]);
   if (first) {
 #pragma unroll
     for (int v = 0; v < 4; ++v) q0bar[v * n + c] = z[v];

@@ -157,7 +157,7 @@ template <class R> __device__ __forceinline__ void forward_update(const Gas<R>& 
   qc[3] = mad(q0[3], g.gamma1, q0[2] * (R(0.5) * u2));  // one contraction, whatever the kernel
 #pragma unroll
   for (int v = 0; v < 4; ++v) qc[v] = mad(tot[v], fac, qc[v]);
-  const St<R> s1 = cons_state(g, qc);
+  const St<R> s1 = cons_state_ir(g, qc, rcp_near(qc[2]));
   qn[0] = s1.u; qn[1] = s1.v; qn[2] = s1.r; qn[3] = s1.p;
 }
 
@@ -633,13 +633,13 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
   R fac;
   if (a.mode == MODE_FUSED_GLOBAL) {
     const R dts = a.beta * R(a.info->dt);
-    fac = div_fast(dts, a.vol[c]);
+    fac = div_near(dts, a.vol[c]);
   } else {
     // local timestep from the stage-0 spectral radius sum (eulerForwardUpdate.h:155-161)
     const R l0 = (a.stage == 0) ? lam : a.res_prev[0][4 * ncell + c];
     const R cs = a.beta * a.cfl;
     // dual time: dtau / (1 + b0 dtau / dt), the physical-time term's share of the spectral radius
-    fac = (DUAL && a.dual_src) ? cs / (l0 + a.cfl * a.vol[c] * a.dual_b0dt) : div_fast(cs, l0);
+    fac = (DUAL && a.dual_src) ? cs / (l0 + a.cfl * a.vol[c] * a.dual_b0dt) : div_near(cs, l0);
   }
   R q0[4], qn[4];
 #pragma unroll
@@ -689,7 +689,7 @@ __device__ __forceinline__ void update0_cell(size_t c, size_t ncell, const Gas<R
     tot[v] = R(0) + alpha00 * res0[v * ncell + c];
     q[v] = q0[v * ncell + c];
   }
-  const R fac = div_fast(dts, vol[c]);
+  const R fac = div_near(dts, vol[c]);
   forward_update(g, q, tot, fac, qn, cons);
 #pragma unroll
   for (int v = 0; v < 4; ++v) q_out[v * ncell + c] = qn[v];

@@ -269,7 +269,7 @@ template <class R> __device__ __forceinline__ void line_cons(const Gas<R>& g, co
   c[2] = mad(q[2], g.gamma1, q[1] * (R(0.5) * (q[0] * q[0])));
 }
 template <class R> __device__ __forceinline__ void line_prim(const Gas<R>& g, const R* c, R* q) {
-  const R ir = rcp_fast(c[1]);
+  const R ir = rcp_near(c[1]);
   q[0] = c[0] * ir;
   q[1] = c[1];
   q[2] = g.gm1 * mad(-c[1], R(0.5) * (q[0] * q[0]), c[2]);
@@ -306,7 +306,7 @@ template <class R, int FK> __global__ void __launch_bounds__(32) stage1d_kernel(
     if (a.stage == 0) a.res_out[3 * n + c] = lam;
   }
   if (a.mode == MODE_RES_MAXRATE || (a.mode == MODE_FUSED_LOCAL && a.norm_stage0 && a.stage == 0)) {
-    R rate = own ? div_fast(lam, G.vol) : R(0);
+    R rate = own ? div_near(lam, G.vol) : R(0);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) rate = max_pos(rate, __shfl_xor_sync(0xffffffffu, rate, o));
     if (lane == 0) atomic_max_rate<R>(a.info, rate);
@@ -326,10 +326,10 @@ template <class R, int FK> __global__ void __launch_bounds__(32) stage1d_kernel(
   for (int v = 0; v < 3; ++v) tot[v] = mad(a.alpha[a.stage], res[v], tot[v]);
   R fac;
   if (a.mode == MODE_FUSED_GLOBAL) {
-    fac = div_fast(a.beta * R(a.info->dt), G.vol);
+    fac = div_near(a.beta * R(a.info->dt), G.vol);
   } else {
     const R l0 = (a.stage == 0) ? lam : a.res_prev[0][3 * n + c];
-    fac = div_fast(a.beta * a.cfl, l0);
+    fac = div_near(a.beta * a.cfl, l0);
   }
   R q0[3], qn[3];
 #pragma unroll
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const _
   const int c = i0 - 1 + min(lane, last);
   const bool own = live && lane >= 1 && lane <= ncell;
   const LineGeom<R> G = line_geom(a.rec, a.vol, nc, per, c);
-  const R ivol = rcp_fast(G.vol);
+  const R ivol = div_near(R(1), G.vol);
   R q[3], qx[3];
   auto load = [&](int k, R* x) {
     const int cc = per ? wrapi(k, nc) : min(max(k, 0), nc - 1);
@@ -467,14 +467,14 @@ __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const _
     const bool final_step = step == a.nsteps - 1;
     // the earlier stages' residuals as their sum: each row of every table weighs them alike
     // (ode.h:107-197)
-    R c0[3], rs[3] = {R(0), R(0), R(0)}, fac0 = R(0);
+    R c0[3], rs[3] = {R(0), R(0), R(0)}, fac0 = R(0), lam0 = R(1);
     line_cons(a.P.gas, q, c0);
 #pragma unroll 1
     for (int s = 0; s < a.nst; ++s) {
       R res[3], lam;
       line_residual<R, FK>(a.P, ref, ghost, G, lane, last, q, qx, s == 0, res, lam);
       if (s == 0) {
-        const R rate = own ? lam * ivol : R(0);
+        const R rate = own ? (sizeof(R) == 4 ? div_near(lam, G.vol) : lam * ivol) : R(0);
         // a NaN or negative rate does not count, as in atomic_max_rate
         const unsigned long long bits =
             rate > R(0) ? (unsigned long long)__double_as_longlong(double(rate)) : 0ull;
@@ -488,10 +488,11 @@ __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const _
           const R dt = R(a.dcfl / r);
           dt_last = double(dt);
           t += dt_last;
-          fac0 = ivol * dt;
+          fac0 = dt;
           if (final_step && tile == 0 && lane == 0) a.info->maxrate = top;
         } else {
-          fac0 = div_fast(a.cfl, lam);
+          fac0 = a.cfl;
+          lam0 = lam;
           if (final_step && lane == 0 && live) atomicMax(&a.info->maxrate, top);
         }
         if (final_step) {
@@ -503,10 +504,13 @@ __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const _
       }
       // rungeKuttaAccumulation (timestepping/rungeKutta.h:172-197) and the update
       R cn[3];
-      const R fac = a.beta[s] * fac0, fs = a.alpha[s][0] * fac, fr = a.alpha[s][s] * fac;
+      // FP64 multiplies by the inverses taken once; FP32 divides, as the launches per stage do
+      const R fac = sizeof(R) == 4 ? div_near(a.beta[s] * fac0, a.global ? G.vol : lam0)
+                                   : (a.beta[s] * fac0) * (a.global ? ivol : rcp_fast(lam0));
 #pragma unroll
       for (int v = 0; v < 3; ++v) {
-        cn[v] = mad(rs[v], s > 0 ? fs : R(0), mad(res[v], fr, c0[v]));
+        const R tot = mad(a.alpha[s][s], res[v], s > 0 ? a.alpha[s][0] * rs[v] : R(0));
+        cn[v] = mad(tot, fac, c0[v]);
         rs[v] = rs[v] + res[v];
       }
       R qn[3];
@@ -568,7 +572,7 @@ __global__ void update0_1d_kernel(int nc, Gas<R> g, const R* __restrict__ q0, co
     R tot[3], q[3], qn[3];
 #pragma unroll
     for (int v = 0; v < 3; ++v) { tot[v] = R(0) + alpha00 * res0[v * n + c]; q[v] = q0[v * n + c]; }
-    update1(g, q, tot, div_fast(beta0 * dt, vol[c]), qn);
+    update1(g, q, tot, div_near(beta0 * dt, vol[c]), qn);
 #pragma unroll
     for (int v = 0; v < 3; ++v) q_out[v * n + c] = qn[v];
     const R chk[4] = {qn[0], R(0), qn[1], qn[2]};

@@ -452,7 +452,7 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
           for (int v = 0; v < 4; ++v) (a.res_out + v * ncell)[cell] = res[v];
           (a.res_out + 4 * ncell)[cell] = lam;
         }
-        rate = fmaxf(rate, qdiv(lam, vol));
+        rate = fmaxf(rate, div_near(lam, vol));
         r2 = fmaf(res[2], res[2], r2);
       } else {
         // rungeKuttaAccumulation (timestepping/rungeKutta.h:172-197): the earlier stages'
@@ -472,16 +472,16 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
             if (a.res_out) (a.res_out + v * ncell)[cell] = res[v];
           }
           if (a.res_out) (a.res_out + 4 * ncell)[cell] = lam;
-          rate = fmaxf(rate, qdiv(lam, vol));
+          rate = fmaxf(rate, div_near(lam, vol));
           r2 = fmaf(res[2], res[2], r2);
         }
         float fac;
         if (a.mode == MODE_FUSED_GLOBAL) {
-          fac = qdiv(a.beta * float(a.info->dt), vol);
+          fac = div_near(a.beta * float(a.info->dt), vol);
         } else {
           // local timestep from the stage-0 spectral radius sum (eulerForwardUpdate.h:155-161)
           const float l0 = sum_in ? pl : lam;
-          fac = qdiv(a.beta * a.cfl, l0);
+          fac = div_near(a.beta * a.cfl, l0);
         }
         float qo[4];
         forward_update(g, pq, tot, fac, qo, false);
