@@ -38,16 +38,18 @@ constexpr int FLUX_BY_TANGENT = -1;
 
 // buffers and recomputation timing shared by the single-mesh and batched drivers
 struct AdjCommon {
-  std::vector<void*> allocs;
+  DevicePool* pool = nullptr;  // the context's or batch's
+  std::vector<std::pair<void*, size_t>> allocs;
   std::vector<cudaEvent_t> adv_events;  // (start, end) pairs around checkpoint recomputation
 
   template <class T> int alloc(T** p, size_t count) {
-    HC_CUDA(cudaMalloc((void**)p, std::max<size_t>(count, 1) * sizeof(T)));
-    allocs.push_back(*p);
+    const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+    HC_CUDA(pool->take((void**)p, bytes));
+    allocs.push_back({*p, bytes});
     return HC_OK;
   }
   ~AdjCommon() {
-    for (void* p : allocs) cudaFree(p);
+    for (auto& a : allocs) pool->give(a.first, a.second);
     for (cudaEvent_t e : adv_events) cudaEventDestroy(e);
   }
   // time of the recorded recomputation segments (call after the stream is idle)
@@ -212,6 +214,7 @@ template <class AD> int alloc_tapes(AD& A, int ntapes, int snapshots) {
     size_t free_b = 0, total_b = 0;
     HC_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t per = size_t(A.nst) * A.state_values() * sizeof(*A.sq[0]);
+    free_b += A.pool->idle_bytes;
     ntapes = int(std::min<size_t>(size_t(snapshots) + 1, free_b / 2 / std::max<size_t>(per, 1)));
   }
   ntapes = std::min(ntapes, A.nsteps);
@@ -219,6 +222,7 @@ template <class AD> int alloc_tapes(AD& A, int ntapes, int snapshots) {
   for (auto& t : A.tapes)
     for (int j = 0; j < A.nst; ++j)
       if (int st = A.alloc(&t.q[j], A.state_values())) return st;
+  A.pool->trim();  // what this recording did not take
   return HC_OK;
 }
 
@@ -617,6 +621,7 @@ template <class R> int setup(Adj<R>& A, hc_ctx* c, int nsteps, int nsnap, const 
   if (int st = ctx_ensure_ready(c)) return st;
   if (int st = check_support(c, obj)) return st;
   A.c = c;
+  A.pool = &c->pool;
   A.nv = c->scalar ? 3 : 4;
   A.tab = rk_table(c->cfg.rk);
   A.nst = A.tab.nst;
@@ -734,6 +739,7 @@ template <class R> int wall_force(hc_ctx* c, const double dir[2], double* out) {
   if (c->cfg.basis != HC_BASIS_PRIMITIVE) return fail(HC_ERR_UNSUPPORTED, "the wall force takes the primitive basis");
   Adj<R> A;
   A.c = c;
+  A.pool = &c->pool;
   A.nv = 4;
   A.n = c->ncell();
   if (int st = A.alloc(&A.qm, 2 * A.state_values())) return st;

@@ -98,6 +98,24 @@ int build_geometry_1d(hc_ctx* c) {
   return HC_OK;
 }
 
+// ghost reference planes in the context precision (2D)
+int upload_refs(hc_ctx* c) {
+  for (int s = 0; s < 4; ++s) {
+    if (c->bc[s] == HC_BC_PERIODIC || c->bc[s] == HC_BC_WALL || c->href[s].empty()) continue;
+    const size_t m = size_t(c->nv) * c->nface(s);
+    if (c->fp32) {
+      std::vector<float> tmp(m);
+      for (size_t k = 0; k < m; ++k) tmp[k] = float(c->href[s][k]);
+      HC_CUDA(cudaMemcpyAsync(c->gref[s], tmp.data(), m * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+      HC_CUDA(cudaStreamSynchronize(c->stream));
+    } else {
+      HC_CUDA(cudaMemcpyAsync(c->gref[s], c->href[s].data(), m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    }
+  }
+  c->gref_dirty = false;
+  return HC_OK;
+}
+
 int build_geometry(hc_ctx* c) {
   if (!c->have_mesh || !c->have_bcs) return fail(HC_ERR_ARG, "mesh and boundary conditions must be set first");
   if (c->oned) return build_geometry_1d(c);
@@ -123,19 +141,7 @@ int build_geometry(hc_ctx* c) {
     c->launches += 2;
   }
   HC_CUDA(cudaGetLastError());
-  // ghost reference planes in the context precision
-  for (int s = 0; s < 4; ++s) {
-    if (c->bc[s] == HC_BC_PERIODIC || c->bc[s] == HC_BC_WALL || c->href[s].empty()) continue;
-    const size_t m = size_t(c->nv) * c->nface(s);
-    if (c->fp32) {
-      std::vector<float> tmp(m);
-      for (size_t k = 0; k < m; ++k) tmp[k] = float(c->href[s][k]);
-      HC_CUDA(cudaMemcpyAsync(c->gref[s], tmp.data(), m * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-      HC_CUDA(cudaStreamSynchronize(c->stream));
-    } else {
-      HC_CUDA(cudaMemcpyAsync(c->gref[s], c->href[s].data(), m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    }
-  }
+  if (int st = upload_refs(c)) return st;
   c->geom_dirty = false;
   return HC_OK;
 }
@@ -144,6 +150,8 @@ int ensure_ready(hc_ctx* c) {
   if (c->geom_dirty) {
     const int st = build_geometry(c);
     if (st != HC_OK) return st;
+  } else if (c->gref_dirty) {
+    if (int st = upload_refs(c)) return st;
   }
   if (!c->have_state) return fail(HC_ERR_ARG, "state not uploaded");
   return HC_OK;
@@ -613,6 +621,7 @@ int hc_context_destroy(hc_ctx* c) {
   if (!c) return HC_OK;
   cudaStreamSynchronize(c->stream);
   c->drop_adj_tape();
+  c->pool.trim();
   free_buffers(c);
   if (c->own) cudaStreamDestroy(c->own);
   delete c;
@@ -640,6 +649,7 @@ int hc_mesh_upload(hc_ctx* c, int ni, int nj, const double* nodes_xy) {
   if (size_t(ni + 1) * size_t(nj + 1) > (size_t(1) << 28)) return fail(HC_ERR_ARG, "mesh too large");
   HC_CUDA(cudaStreamSynchronize(c->stream));
   c->drop_adj_tape();
+  c->pool.trim();
   free_buffers(c);
   c->oned = false;
   c->nv = c->scalar ? 3 : 4;
@@ -694,6 +704,7 @@ int hc_mesh_upload_1d(hc_ctx* c, int nc, const double* nodes_x) {
     if (!(nodes_x[i + 1] > nodes_x[i])) return fail(HC_ERR_ARG, "1D nodes must increase");
   HC_CUDA(cudaStreamSynchronize(c->stream));
   c->drop_adj_tape();
+  c->pool.trim();
   free_buffers(c);
   c->oned = true;
   c->nv = 3;
@@ -810,6 +821,9 @@ int hc_set_bcs(hc_ctx* c, const int bc_type[4], const double* const ref[4]) {
   if ((bc_type[0] == HC_BC_PERIODIC) != (bc_type[1] == HC_BC_PERIODIC) ||
       (bc_type[2] == HC_BC_PERIODIC) != (bc_type[3] == HC_BC_PERIODIC))
     return fail(HC_ERR_ARG, "periodic sides must come in pairs (0,1) and (2,3)");
+  // the geometry depends on the boundary types alone
+  bool same = c->have_bcs;
+  for (int s = 0; s < 4; ++s) same = same && c->bc[s] == bc_type[s];
   for (int s = 0; s < 4; ++s) {
     c->bc[s] = bc_type[s];
     c->href[s].clear();
@@ -820,7 +834,8 @@ int hc_set_bcs(hc_ctx* c, const int bc_type[4], const double* const ref[4]) {
     }
   }
   c->have_bcs = true;
-  c->geom_dirty = true;
+  if (same) c->gref_dirty = true;
+  else c->geom_dirty = true;
   return HC_OK;
 }
 

@@ -358,6 +358,7 @@ int hc_batch_destroy(hc_batch* b) {
   if (!b) return HC_OK;
   cudaStreamSynchronize(b->stream);
   b->drop_adj_tape();
+  b->pool.trim();
   free_all(b);
   if (b->own) cudaStreamDestroy(b->own);
   delete b;

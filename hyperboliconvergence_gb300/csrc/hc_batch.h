@@ -55,6 +55,8 @@ struct hc_batch {
     adj_tape = nullptr;
   }
 
+  hc::DevicePool pool;  // the adjoint's blocks between two gradients
+
   size_t icells(int k) const { return size_t(ni[k]) * nj[k]; }
 };
 

@@ -329,6 +329,7 @@ int batch_setup(BAdj<R>& A, hc_batch* b, int nsteps, int nsnap, const hc_objecti
     if (!targets[k]) return fail(HC_ERR_ARG, "instance " + std::to_string(k) + " has no target");
   if (int st = check_batch_support(b)) return st;
   A.b = b;
+  A.pool = &b->pool;
   A.ninst = b->ninst;
   A.tab = rk_table(b->cfg.rk);
   A.nst = A.tab.nst;
@@ -374,12 +375,16 @@ int batch_setup(BAdj<R>& A, hc_batch* b, int nsteps, int nsnap, const hc_objecti
   HC_CUDA(cudaMemsetAsync(A.jacc, 0, A.ninst * sizeof(double), A.s()));
   if (int st = A.alloc(&A.part, A.n)) return st;
   if (int st = A.alloc(&A.target, n4)) return st;
-  // targets through the batch's FP64 staging buffer (one instance at a time)
+  // host targets through the batch's FP64 staging buffer (one instance at a time)
   if (b->scalar) HC_CUDA(cudaMemsetAsync(A.target, 0, n4 * sizeof(R), A.s()));
   for (int k = 0; k < A.ninst; ++k) {
     const size_t m = size_t(b->nv) * b->icells(k);
-    HC_CUDA(cudaMemcpyAsync(b->staging, targets[k], m * sizeof(double),
-                            obj->target_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, A.s()));
+    if (obj->target_on_device) {
+      convert_kernel<R><<<512, 256, 0, A.s()>>>(targets[k], A.target + 4 * b->cell_off[k], m);
+      HC_CUDA(cudaGetLastError());
+      continue;
+    }
+    HC_CUDA(cudaMemcpyAsync(b->staging, targets[k], m * sizeof(double), cudaMemcpyHostToDevice, A.s()));
     convert_kernel<R><<<512, 256, 0, A.s()>>>(b->staging, A.target + 4 * b->cell_off[k], m);
     HC_CUDA(cudaGetLastError());
     HC_CUDA(cudaStreamSynchronize(A.s()));  // targets[k] and the staging buffer are reused

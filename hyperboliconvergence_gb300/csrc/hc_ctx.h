@@ -33,6 +33,8 @@ struct hc_ctx {
     if (adj_tape && adj_tape_free) adj_tape_free(adj_tape);
     adj_tape = nullptr;
   }
+  hc::DevicePool pool;                              // the adjoint's blocks between two gradients
+  bool gref_dirty = false;                          // new reference values, same boundary types
   void* dual_src = nullptr;                         // dual time: earlier levels' terms (4 planes, R)
   double dual_g0 = 1.0, dual_b0dt = 0.0;            // dual time: gamma_0 and beta_0 / dt
   double smooth_alpha = 0.0;                        // 1D residual smoothing factor (0: off)
