@@ -295,7 +295,8 @@ template <class R> int run_line(hc_ctx* c, int nsteps) {
   while (nsteps > 0) {
     a.nsteps = std::min(nsteps, kLineChunk);
     nsteps -= a.nsteps;
-    HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
+    if (!c->words_clear) HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
+    c->words_clear = false;
     HC_CUDA(launch_line_run<R>(a, c->cfg.flux, c->stream));
     c->launches += 1;
   }
@@ -315,7 +316,10 @@ template <class R> int run_residual(hc_ctx* c) {
 }
 
 // One RK step: the stage loop of integrate() (timestepping/rungeKutta.h:97-164).
-template <class R> int run_step(hc_ctx* c) {
+// first: the call's first step (its words are clear); last: its last one, whose maximum rate and
+// norm are read.  In between, each step's last stage clears the words of the next, and the
+// kernels follow one another by chained launches.
+template <class R> int run_step(hc_ctx* c, bool first = false, bool last = true) {
   if (c->oned) return run_step_1d<R>(c);
   const RKTab tab = rk_table(c->cfg.rk);
   const int nst = tab.nst;
@@ -324,7 +328,11 @@ template <class R> int run_step(hc_ctx* c) {
   auto fn = [c, euler_fn](const StageArgs<R>& a, int tile, cudaStream_t s) -> cudaError_t {
     return c->scalar ? launch_scalar_stage<R>(a, c->cfg.flux, tile, s) : euler_fn(a, tile, s);
   };
-  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
+  // a table of one stage has no later stage to clear the words; the scalar law's kernels neither
+  // chain nor clear
+  const bool chain = nst > 1 && !c->scalar;
+  if (!chain || !c->words_clear) HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kStepWords, c->stream));
+  c->words_clear = false;
   auto out_of = [&](int s) -> R* { return (R*)((s == nst - 1) ? c->q[0] : c->q[1 + (s % 2)]); };
   for (int s = 0; s < nst; ++s) {
     StageArgs<R> a = base_args<R>(c);
@@ -335,6 +343,8 @@ template <class R> int run_step(hc_ctx* c) {
     for (int k = 0; k < s; ++k) a.res_prev[k] = (const R*)c->res[k];
     a.res_out = (s < nst - 1) ? (R*)c->res[s] : nullptr;
     a.norm_stage0 = (s == 0);
+    a.chained = chain && !(first && s == 0);
+    a.clear_words = chain && !last && s == nst - 1;
     if (global && s == 0) {
       a.mode = MODE_RES_MAXRATE;
       a.res_out = (R*)c->res[0];
@@ -347,10 +357,10 @@ template <class R> int run_step(hc_ctx* c) {
                                          R(tab.alpha[0][0]), R(tab.beta[0]), c->cfg.cfl, c->info, out_of(0), 1,
                                          c->stream));
       } else {
-        update0_kernel<R><<<grid, B, 0, c->stream>>>(c->ni, c->nj, a.gas, (const R*)c->q[0], (const R*)c->res[0],
-                                                     (const R*)c->vol, R(tab.alpha[0][0]), R(tab.beta[0]),
-                                                     c->cfg.cfl, c->info, out_of(0), 1, c->cfg.basis,
-                                                     c->dual_src ? c->dual_b0dt : 0.0);
+        HC_CUDA(launch_chained(update0_kernel<R>, dim3(grid), B, 0, c->stream, chain, c->ni, c->nj, a.gas,
+                               (const R*)c->q[0], (const R*)c->res[0], (const R*)c->vol, R(tab.alpha[0][0]),
+                               R(tab.beta[0]), c->cfg.cfl, c->info, out_of(0), 1, c->cfg.basis,
+                               c->dual_src ? c->dual_b0dt : 0.0));
       }
       HC_CUDA(cudaGetLastError());
       c->launches += 2;
@@ -361,6 +371,7 @@ template <class R> int run_step(hc_ctx* c) {
       c->launches += 1;
     }
   }
+  c->words_clear = chain && !last;
   return HC_OK;
 }
 
@@ -536,7 +547,7 @@ template <class R> int dual_time_run(hc_ctx* c, const hc_dual_time_controls* ctl
     while (m < ctl->inner_max) {
       const int chunk = (m == 0) ? 1 : std::min(ctl->check_every, ctl->inner_max - m);
       for (int j = 0; j < chunk; ++j)
-        if (int e = run_step<R>(c)) return e;
+        if (int e = run_step<R>(c, j == 0, j == chunk - 1)) return e;
       m += chunk;
       hc_step_stats s{};
       if (int e = read_stats(c, &s)) return e;
@@ -933,14 +944,17 @@ int hc_step_async(hc_ctx* c, int nsteps) {
   if (int st = check_ctx(c)) return st;
   if (nsteps < 0) return fail(HC_ERR_ARG, "negative step count");
   if (int st = ensure_ready(c)) return st;
-  // clear the device status of earlier calls (status and bad_cell are adjacent ints)
-  HC_CUDA(cudaMemsetAsync(&c->info->status, 0, 2 * sizeof(int), c->stream));
+  // clear the device status of earlier calls, and the first step's words
+  HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kCallWords, c->stream));
+  c->words_clear = true;
   if (c->oned && c->ni <= kLineMax && !(c->smooth_alpha > 0.0))
     return c->fp32 ? run_line<float>(c, nsteps) : run_line<double>(c, nsteps);
   for (int k = 0; k < nsteps; ++k) {
-    const int st = c->fp32 ? run_step<float>(c) : run_step<double>(c);
-    if (st != HC_OK) return st;
+    const bool first = k == 0, last = k == nsteps - 1;
+    const int st = c->fp32 ? run_step<float>(c, first, last) : run_step<double>(c, first, last);
+    if (st != HC_OK) { c->words_clear = false; return st; }
   }
+  c->words_clear = false;
   return HC_OK;
 }
 

@@ -34,6 +34,7 @@ struct hc_ctx {
     adj_tape = nullptr;
   }
   hc::DevicePool pool;                              // the adjoint's blocks between two gradients
+  bool words_clear = false;                         // the next step's maximum rate and norm are clear
   bool gref_dirty = false;                          // new reference values, same boundary types
   void* dual_src = nullptr;                         // dual time: earlier levels' terms (4 planes, R)
   double dual_g0 = 1.0, dual_b0dt = 0.0;            // dual time: gamma_0 and beta_0 / dt

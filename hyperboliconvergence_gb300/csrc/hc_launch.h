@@ -85,6 +85,24 @@ template <class R>
 cudaError_t launch_scalar_batch_update0(const BatchArgs<R>& b, int tile, int grid, double cfl, R alpha00, R beta0,
                                         cudaStream_t s);
 
+// a launch behind the kernel before it on the stream, its blocks waiting in chain_wait
+// (chained), or an ordinary one
+template <class K, class... A>
+inline cudaError_t launch_chained(K* kernel, dim3 grid, unsigned threads, size_t smem, cudaStream_t s, bool chained,
+                                  const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // the strip kernel's arguments of one mesh
 inline StripArgs strip_args(const StageArgs<float>& a) {
   StripArgs p{};
@@ -143,7 +161,7 @@ inline void tile_dims(int tile, int* ti, int* tj) {
   template <int LIM> static bool go_strip(const StageArgs<float>& a, cudaStream_t s) {                  \
     const StripArgs p = strip_args(a);                                                                  \
     const unsigned grid = unsigned((p.strips * p.runs + kStripWarps - 1) / kStripWarps);                \
-    strip_kernel<FK, LIM><<<grid, 32 * kStripWarps, kStripSmem, s>>>(p);                                \
+    launch_chained(strip_kernel<FK, LIM>, dim3(grid), 32 * kStripWarps, kStripSmem, s, a.chained != 0, p); \
     return true;                                                                                        \
   }                                                                                                     \
   static bool go_strips(const StageArgs<float>& a, cudaStream_t s) {                                    \
@@ -209,7 +227,8 @@ inline void tile_dims(int tile, int* ti, int* tj) {
   }                                                                                                      \
   template <class R, int TI, int TJ> static void go(const StageArgs<R>& a, cudaStream_t s) {             \
     const dim3 grid((a.nj + TJ - 1) / TJ, (a.ni + TI - 1) / TI);                                         \
-    stage_kernel<TI, TJ, R, FK><<<grid, TI * TJ, StageSmem<TI, TJ, R>::bytes, s>>>(a);                   \
+    launch_chained(stage_kernel<TI, TJ, R, FK>, grid, TI * TJ, StageSmem<TI, TJ, R>::bytes, s,           \
+                   a.chained != 0, a);                                                                   \
   }                                                                                                      \
   template <class R> static cudaError_t prep_half() {                                                   \
     return cudaFuncSetAttribute(stage_kernel<16, 16, R, FK, R, 128>,                                     \
@@ -235,9 +254,9 @@ inline void tile_dims(int tile, int* ti, int* tj) {
     if (std::is_same<R, double>::value && a.fic) {                                                       \
       /* double-float compute type, 8x32 tiles */                                                        \
       const dim3 grid((a.nj + 31) / 32, (a.ni + 7) / 8);                                                 \
-      stage_kernel<8, 32, double, FK, df64><<<grid, 256, StageSmem<8, 32, df64>::bytes, s>>>(           \
-          *reinterpret_cast<const StageArgs<double>*>(&a));                                              \
-      return cudaGetLastError();                                                                         \
+      return launch_chained(stage_kernel<8, 32, double, FK, df64>, grid, 256,                           \
+                            StageSmem<8, 32, df64>::bytes, s, a.chained != 0,                            \
+                            *reinterpret_cast<const StageArgs<double>*>(&a));                            \
     }                                                                                                    \
     if constexpr (std::is_same<R, float>::value) {                                                       \
       if ((tile == TILE_8x32 || tile < 0 || tile >= TILE_COUNT) && go_strips(a, s)) return cudaGetLastError(); \
@@ -246,20 +265,21 @@ inline void tile_dims(int tile, int* ti, int* tj) {
       if (tile == TILE_AUTO) tile = f64_auto_tile(a.ni, a.nj);                                           \
       if (tile == TILE_8x8) {                                                                            \
         const dim3 grid((a.nj + 7) / 8, (a.ni + 7) / 8);                                                 \
-        stage_kernel<8, 8, R, FK, R, 160><<<grid, 160, StageSmem<8, 8, R>::bytes, s>>>(a);               \
-        return cudaGetLastError();                                                                       \
+        return launch_chained(stage_kernel<8, 8, R, FK, R, 160>, grid, 160, StageSmem<8, 8, R>::bytes, s, \
+                              a.chained != 0, a);                                                        \
       }                                                                                                  \
       if (tile == TILE_4x8) {                                                                            \
         const dim3 grid((a.nj + 7) / 8, (a.ni + 3) / 4);                                                 \
-        stage_kernel<4, 8, R, FK, R, 96><<<grid, 96, StageSmem<4, 8, R>::bytes, s>>>(a);                 \
-        return cudaGetLastError();                                                                       \
+        return launch_chained(stage_kernel<4, 8, R, FK, R, 96>, grid, 96, StageSmem<4, 8, R>::bytes, s,  \
+                              a.chained != 0, a);                                                        \
       }                                                                                                  \
     }                                                                                                    \
     if (tile == TILE_4x32) go<R, 4, 32>(a, s);                                                           \
     else if (tile == TILE_16x16) go<R, 16, 16>(a, s);                                                    \
     else if (tile == TILE_16x16_H) {                                                                     \
       const dim3 grid((a.nj + 15) / 16, (a.ni + 15) / 16);                                               \
-      stage_kernel<16, 16, R, FK, R, 128><<<grid, 128, StageSmem<16, 16, R>::bytes, s>>>(a);             \
+      return launch_chained(stage_kernel<16, 16, R, FK, R, 128>, grid, 128, StageSmem<16, 16, R>::bytes, s, \
+                            a.chained != 0, a);                                                          \
     } else go<R, 8, 32>(a, s);                                                                           \
     return cudaGetLastError();                                                                           \
   }                                                                                                      \

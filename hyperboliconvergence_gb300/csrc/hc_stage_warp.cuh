@@ -249,6 +249,8 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
   fetch_row(r0 - 1, false);
   fetch_row(r0, a.stall_copy != 0);
 
+  // the records do not depend on the stage before: their copies are under way while it ends
+  chain_wait<true>();
   float qa[4], qb[4], qc[4], qn[4];  // rows r, r + 1, r + 2, r + 3
   {
     const unsigned k0 = qcell(r0 - 2), k1 = qcell(r0 - 1), k2 = qcell(r0), k3 = qcell(r0 + 1);
@@ -541,6 +543,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, 4) strip_kernel(const StripA
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int item = int(blockIdx.x) * kStripWarps + int(threadIdx.x >> 5);
   if (item >= p.strips * p.runs) return;
+  if (p.a.clear_words && item == 0 && threadIdx.x == 0) chain_wait<true>();
+  clear_step_words(p.a);
   StripRing ring = strip_ring(smem_raw, !p.a.plain_loads);
   const int w = item % p.strips, r0 = (item / p.strips) * p.rows;
   strip_run<FK, LIM>(p.a, p.a.pk, w, r0, min(r0 + p.rows, p.a.ni), ring);
