@@ -75,7 +75,7 @@ int build_worklist(hc_batch* b) {
   if (b->pk) {
     b->strip_rows = strip_run_rows(b->ninst, [&](int k) { return b->ni[k]; }, [&](int k) { return b->nj[k]; }, b->sms);
     for (int k : perm) {
-      const int nt = strip_count(b->nj[k]) * ((b->ni[k] + b->strip_rows - 1) / b->strip_rows);
+      const int nt = strip_count(b->nj[k]) * strip_runs(b->ni[k], b->strip_rows);
       if (nt > 0xffff) return fail(HC_ERR_UNSUPPORTED, "instance has more than 65535 strips");
       for (int t = 0; t < nt; ++t) strips.push_back((k << 16) | t);
     }

@@ -103,13 +103,17 @@ inline cudaError_t launch_chained(K* kernel, dim3 grid, unsigned threads, size_t
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// whether the strip kernel takes an FP32 launch of the 8 x 32 tile
+inline bool strips_take(const float* pk, int basis, int limiter) {
+  return pk && basis == 0 && (limiter == LIM_VANALBADA || limiter == LIM_VANLEER || limiter == LIM_MINMOD ||
+                              limiter == LIM_NOLIMIT2 || limiter == LIM_NOLIMIT3);
+}
 // the strip kernel's arguments of one mesh
 inline StripArgs strip_args(const StageArgs<float>& a) {
   StripArgs p{};
   p.a = a;
   p.strips = strip_count(a.nj);
-  p.rows = strip_run_rows(1, [&](int) { return a.ni; }, [&](int) { return a.nj; }, device_sms());
-  p.runs = (a.ni + p.rows - 1) / p.rows;
+  p.runs = strip_runs(a.ni, strip_run_rows(1, [&](int) { return a.ni; }, [&](int) { return a.nj; }, device_sms()));
   return p;
 }
 
@@ -165,7 +169,7 @@ inline void tile_dims(int tile, int* ti, int* tj) {
     return true;                                                                                        \
   }                                                                                                     \
   static bool go_strips(const StageArgs<float>& a, cudaStream_t s) {                                    \
-    if (!a.pk || a.basis != 0 || a.dual_src) return false;                                              \
+    if (!strips_take(a.pk, a.basis, a.limiter) || a.dual_src) return false;                             \
     switch (a.limiter) {                                                                                \
       case LIM_VANALBADA: return go_strip<LIM_VANALBADA>(a, s);                                         \
       case LIM_VANLEER: return go_strip<LIM_VANLEER>(a, s);                                             \
@@ -180,7 +184,7 @@ inline void tile_dims(int tile, int* ti, int* tj) {
     return true;                                                                                        \
   }                                                                                                     \
   static bool gob_strips(const BatchArgs<float>& b, cudaStream_t s) {                                   \
-    if (!b.pk || b.basis != 0) return false;                                                            \
+    if (!strips_take(b.pk, b.basis, b.limiter)) return false;                                           \
     switch (b.limiter) {                                                                                \
       case LIM_VANALBADA: return gob_strip<LIM_VANALBADA>(b, s);                                        \
       case LIM_VANLEER: return gob_strip<LIM_VANLEER>(b, s);                                            \

@@ -59,29 +59,31 @@ __host__ __device__ inline size_t strip_floats(int ni, int nj) {
   return size_t(strip_count(nj)) * (ni + kStripRowsBefore) * kStripRow;
 }
 
-// Rows of a run for the given meshes: the launch takes the waves its runs make of the 152 SMs'
-// resident warps, times a run's rows and its lead-in (1.7 rows' work); small meshes are cut
-// finer, so that every SM has work.  512 x 1024, ms per step: 8 rows 0.115, 16 rows 0.24 (half a
-// wave: each warp's latency is exposed).
+// Rows of a run, at most, for the given meshes (a mesh's rows are divided evenly over
+// ceil(ni / rows) runs): a launch takes the waves its runs make of the 152 SMs' resident warps,
+// times a run's rows and its lead-in (1.7 rows' work).  Small meshes are cut finer, so that
+// every SM has work, and large ones so that the last wave is full.  Measured, ms per step: 512 x
+// 1024 with 8 rows (one wave) 0.115, with 16 (half a wave: each warp's latency is exposed) 0.24;
+// a batch of 24 meshes, 2.27 M cells, with 8 rows (4.2 waves) 0.64, by this rule (2 waves) 0.57;
+// 96 small ones, 0.47 M cells, 0.255 and 0.20.
+inline int strip_runs(int ni, int rows) { return (ni + rows - 1) / rows; }
 template <class NI, class NJ> inline int strip_run_rows(int n, NI ni, NJ nj, int sms) {
   constexpr int kResident = 16;  // warps per SM
-  static const int cand[] = {1, 2, 3, 4, 6, 8, 10, 12, 16, 20, 24, 32};
-  int best = 32;
+  int best = 1;
   double cost = 1e300;
-  for (int rows : cand) {
+  for (int rows = 1; rows <= 64; ++rows) {
     long long items = 0;
+    int longest = 0;
     bool fits = true;  // a work item is packed in 16 bits within its instance
     for (int k = 0; k < n; ++k) {
-      const long long m = (long long)strip_count(nj(k)) * ((ni(k) + rows - 1) / rows);
+      const int runs = strip_runs(ni(k), rows);
+      const long long m = (long long)strip_count(nj(k)) * runs;
       items += m;
+      longest = std::max(longest, (ni(k) + runs - 1) / runs);
       fits = fits && (n == 1 || m <= 0xffff);
     }
-    if (!fits) continue;
-    // up to one wave of resident warps takes a wave's time, then whole waves, then the average
-    const double waves = double(items) / (double(sms) * kResident);
-    const double w = waves > 4 ? waves : std::ceil(waves);
-    const double c = w * (rows + 1.7);
-    if (c < cost) { cost = c; best = rows; }
+    const double c = std::ceil(double(items) / (double(sms) * kResident)) * (longest + 1.7);
+    if (fits && c < cost) { cost = c; best = rows; }
   }
   return best;
 }
@@ -94,7 +96,7 @@ cudaError_t pack_strips(const double* fi, const double* fj, const double* vol, i
 
 struct StripArgs {
   StageArgs<float> a;
-  int strips, runs, rows;  // strips of the mesh, runs of rows, rows of a run
+  int strips, runs;  // strips of the mesh, runs of rows
 };
 
 // ---- limiters on arguments scaled by the centres' distance
@@ -520,6 +522,9 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
   }
 }
 
+// first row of a run
+__device__ __forceinline__ int strip_row(int ni, int run, int runs) { return int((long long)ni * run / runs); }
+
 // the warp's ring in the block's shared memory, its barriers initialised
 __device__ __forceinline__ StripRing strip_ring(unsigned char* smem, bool staged) {
   const int warp = threadIdx.x >> 5;
@@ -546,12 +551,14 @@ __global__ void __launch_bounds__(32 * kStripWarps, 4) strip_kernel(const StripA
   if (p.a.clear_words && item == 0 && threadIdx.x == 0) chain_wait<true>();
   clear_step_words(p.a);
   StripRing ring = strip_ring(smem_raw, !p.a.plain_loads);
-  const int w = item % p.strips, r0 = (item / p.strips) * p.rows;
-  strip_run<FK, LIM>(p.a, p.a.pk, w, r0, min(r0 + p.rows, p.a.ni), ring);
+  const int w = item % p.strips, run = item / p.strips;
+  strip_run<FK, LIM>(p.a, p.a.pk, w, strip_row(p.a.ni, run, p.runs), strip_row(p.a.ni, run + 1, p.runs), ring);
 }
 
 // The strips of every instance of a batch: the warps of a persistent grid walk the work list
-// (b.strip_order, packed instance << 16 | run * strips + strip).
+// (b.strip_order, packed instance << 16 | run * strips + strip).  Its launches are not chained:
+// a block that starts early while others of the kernel before still run upsets the even split
+// of the list (24 meshes, 20 steps from a graph: 12.5 ms chained, 11.4 not).
 template <int FK, int LIM>
 __global__ void __launch_bounds__(32 * kStripWarps, 4) batch_strip_kernel(const __grid_constant__ BatchArgs<float> b) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -565,8 +572,8 @@ __global__ void __launch_bounds__(32 * kStripWarps, 4) batch_strip_kernel(const 
     __syncwarp();
     const StageArgs<float>& a = sa[warp];
     const int strips = strip_count(a.nj);
-    const int w = t % strips, r0 = (t / strips) * b.strip_rows;
-    strip_run<FK, LIM>(a, a.pk, w, r0, min(r0 + b.strip_rows, a.ni), ring);
+    const int w = t % strips, run = t / strips, runs = (a.ni + b.strip_rows - 1) / b.strip_rows;
+    strip_run<FK, LIM>(a, a.pk, w, strip_row(a.ni, run, runs), strip_row(a.ni, run + 1, runs), ring);
     __syncwarp();
   }
 }
