@@ -15,18 +15,22 @@
 // shared memory while the two rows before it are computed, whatever the mesh's width.  The
 // waits are bounded (a copy that never lands marks the step ST_TIMEOUT).  The records hold the
 // limiter's arguments scaled by the distance between the cell centres, w (dl + dr),
-// s (dl + dr), dl/(dl + dr) and dr/(dl + dr): the limiters are homogeneous, and the division
+// -s (dl + dr), dl/(dl + dr) and -dr/(dl + dr): the limiters are homogeneous, and the division
 // by that distance disappears.
 //
-// What bounds it: instruction issue (59% of the issue slots at four warps per scheduler, no pipe
-// above 30%; 1,190 thread instructions per cell and stage, halo lanes and lead-in rows
-// included).  The tiled kernel before it (8 x 32 cells, halo and gradient tiles in shared
-// memory, four block barriers) issued 1,577 at 45%, waiting on barriers and on the j-face
-// records.  512 x 1024 O-grid, Roe + van Albada: 0.168 -> 0.115 ms per ssp34 step; a batch of 24
-// uneven quadrant problems, SLAU, 20 steps, uploads and downloads included: 18.8 -> 15.8 ms.
-// Four blocks of four warps per SM: 126 registers hold a pass without spills (with the edge
-// faces' code out of line the calls cost 48 bytes of spills and 15% of the time), and 512 x 1024
-// in runs of 8 rows is one wave of 2,368 warps.
+// What bounds it: instruction issue (60% of the issue slots at four warps per scheduler, no pipe
+// above 30%; 834 instructions per warp and row).  So what comes in twos -- a face's left and
+// right side, a gradient's x and y -- is computed as packed FP32 pairs, one instruction for two
+// operations, from records that hold the pairs side by side, and the planes are addressed by a
+// 32-bit byte offset that serves all of them: 912 instructions before, 512 x 1024 O-grid, Roe +
+// van Albada: 0.104 -> 0.096 ms per ssp34 step, 301 x 715, AUSM+up + van Leer: 0.062 -> 0.059.
+// The tiled kernel before the strips (8 x 32 cells, halo and gradient tiles in shared memory,
+// four block barriers) issued a third more at 45%, waiting on barriers and on the j-face records:
+// 0.174 and 0.100 ms; a batch of 24 uneven quadrant problems, SLAU, 20 steps, uploads and downloads
+// included: 18.8 ms, now 14.7.
+// Four blocks of four warps per SM: at most 128 registers, which hold a pass without spills (with
+// the edge faces' code out of line the calls cost 48 bytes of spills and 15% of the time), and
+// 512 x 1024 in runs of 8 rows is one wave of 2,368 warps.
 //
 // The stage residuals of the alpha/beta tables are kept as their running sum (each row of every
 // table weighs the earlier stages alike, ode.h:107-197), so a later stage reads and writes one
@@ -42,12 +46,15 @@ namespace hc {
 
 constexpr int kStripCells = 28;                      // columns a strip owns
 constexpr int kStripRowsBefore = 3;                  // record rows before row 0 (the run's lead-in)
-// fields of a record row r, in the order of the first and last rows' needs: the gradient sums of
-// row r + 1 (left j-face and lower i-face offsets), the i-face r + 1, the volume of row r, the
-// j-face on the left of row r + 1
+// A record row r, in units of 32 floats and in the order of the first and last rows' needs: the
+// gradient sums of row r + 1 (left j-face and lower i-face offsets), the i-face r + 1, the
+// volume of row r, the j-face on the left of row r + 1.
 enum StripField { S_DXJ = 0, S_DXI = 2, S_IF = 4, S_VOL = 15, S_JF = 16, S_FIELDS = 27 };
-// fields of a face within S_IF / S_JF
-enum StripFace { P_NX = 0, P_NY, P_A, P_CL, P_CR, P_WLX, P_WLY, P_SL, P_WRX, P_WRY, P_SR, P_FIELDS };
+// Fields of a face within S_IF / S_JF, likewise.  All but the area are pairs, a lane's two
+// values side by side: the weights of the face's left and right side (of a j-face: of the cell's
+// right face as its left side, and of its left face as its right side, so that both are the
+// lane's own cell's), the sums' factors -s and the distances cl, -cr alike, and the normal.
+enum StripFace { P_WX = 0, P_WY = 2, P_S = 4, P_C = 6, P_N = 8, P_A = 10, P_FIELDS = 11 };
 constexpr int kStripRow = S_FIELDS * 32;             // floats of one strip and row
 constexpr int kStripSlots = 3;
 constexpr int kStripWarps = 4;                       // warps of a block
@@ -63,7 +70,7 @@ __host__ __device__ inline size_t strip_floats(int ni, int nj) {
 // ceil(ni / rows) runs): a launch takes the waves its runs make of the 152 SMs' resident warps,
 // times a run's rows and its lead-in (1.7 rows' work).  Small meshes are cut finer, so that
 // every SM has work, and large ones so that the last wave is full.  Measured, ms per step: 512 x
-// 1024 with 8 rows (one wave) 0.115, with 16 (half a wave: each warp's latency is exposed) 0.24;
+// 1024 with 8 rows (one wave) 0.104, with 16 (half a wave: each warp's latency is exposed) 0.21;
 // a batch of 24 meshes, 2.27 M cells, with 8 rows (4.2 waves) 0.64, by this rule (2 waves) 0.57;
 // 96 small ones, 0.47 M cells, 0.255 and 0.20.
 inline int strip_runs(int ni, int rows) { return (ni + rows - 1) / rows; }
@@ -99,12 +106,59 @@ struct StripArgs {
   int strips, runs;  // strips of the mesh, runs of rows
 };
 
+// ---- pairs of FP32 values: one instruction for two operations (FFMA2 and its kin run at the
+// rate of two FP32 instructions but take one issue slot, which is what bounds the kernel)
+struct f2 { unsigned long long v; };
+__device__ __forceinline__ f2 pair(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float lo(f2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return x;
+}
+__device__ __forceinline__ float hi(f2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+  return y;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+// Value at a byte offset of 32 bits from a plane's base (the same in every lane, so that one
+// address register serves all planes).
+__device__ __forceinline__ float at(const float* plane, unsigned off) {
+  return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(plane) + off);
+}
+__device__ __forceinline__ float& at(float* plane, unsigned off) {
+  return *reinterpret_cast<float*>(reinterpret_cast<char*>(plane) + off);
+}
+// a lane's pair of a record field
+__device__ __forceinline__ f2 pair_at(const float* p) {
+  f2 r;
+  r.v = *reinterpret_cast<const unsigned long long*>(p);
+  return r;
+}
+
 // ---- limiters on arguments scaled by the centres' distance
 template <int LIM> __device__ __forceinline__ float strip_limit(float a, float b) {
   if constexpr (LIM == LIM_VANALBADA) {
-    const float ab = a * b;
-    const float s = (ab * (a + b)) * rcp_f32(fmaf(a, a, fmaf(b, b, FLT_MIN)));
-    return ab <= 0.f ? 0.f : s;
+    const float ab = fmaxf(a * b, 0.f);  // 0 slope where a b <= 0; a NaN comes back with a + b
+    return (ab * (a + b)) * rcp_f32(fmaf(b, b, fmaf(a, a, FLT_MIN)));
   } else if constexpr (LIM == LIM_VANLEER) {
     const float ab = a * b;
     const float s = (ab + ab) * rcp_f32(a + b);
@@ -112,6 +166,31 @@ template <int LIM> __device__ __forceinline__ float strip_limit(float a, float b
   } else {
     return limit<float>(LIM, a, b);
   }
+}
+template <int LIM> __device__ __forceinline__ f2 strip_limit2(f2 a, f2 b) {
+  if constexpr (LIM == LIM_VANALBADA) {
+    const f2 t = mul2(a, b);
+    const f2 ab = pair(fmaxf(lo(t), 0.f), fmaxf(hi(t), 0.f));
+    const f2 den = fma2(b, b, fma2(a, a, pair(FLT_MIN, FLT_MIN)));
+    return mul2(mul2(ab, add2(a, b)), pair(rcp_f32(lo(den)), rcp_f32(hi(den))));
+  } else if constexpr (LIM == LIM_VANLEER) {
+    const f2 ab = mul2(a, b), sum = add2(a, b);
+    const f2 s = mul2(add2(ab, ab), pair(rcp_f32(lo(sum)), rcp_f32(hi(sum))));
+    return pair(lo(ab) <= 0.f ? 0.f : lo(s), hi(ab) <= 0.f ? 0.f : hi(s));
+  } else {
+    return pair(strip_limit<LIM>(lo(a), lo(b)), strip_limit<LIM>(hi(a), hi(b)));
+  }
+}
+// the two states of a face from the pairs {left, right} of its primitive values (prim_state_ir)
+__device__ __forceinline__ void strip_states(const Gas<float>& g, const f2* q, St<float>& l, St<float>& r) {
+  const f2 ir = pair(rcp_f32(lo(q[2])), rcp_f32(hi(q[2])));
+  const f2 u2 = fma2(q[1], q[1], mul2(q[0], q[0]));
+  const f2 a2 = mul2(pair(g.gamma, g.gamma), mul2(q[3], ir));
+  const f2 h = fma2(a2, pair(g.gamma1, g.gamma1), mul2(pair(0.5f, 0.5f), u2));
+  l.u = lo(q[0]); l.v = lo(q[1]); l.r = lo(q[2]); l.p = lo(q[3]);
+  l.u2 = lo(u2); l.ir = lo(ir); l.a2 = lo(a2); l.h = lo(h);
+  r.u = hi(q[0]); r.v = hi(q[1]); r.r = hi(q[2]); r.p = hi(q[3]);
+  r.u2 = hi(u2); r.ir = hi(ir); r.a2 = hi(a2); r.h = hi(h);
 }
 
 // Flux through a non-periodic boundary face: wall, or a ghost state on the far side (fixed,
@@ -233,12 +312,12 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
   const Gas<float>& g = a.gas;
   const float* rows = pk + size_t(w) * (ni + kStripRowsBefore) * kStripRow;  // record row r at (r + 3) kStripRow
   auto recrow = [&](int r) { return rows + size_t(r + kStripRowsBefore) * kStripRow; };
-  // the lane's cell in row r (fewer than 2^28 cells: 32-bit offsets from the planes' bases)
+  // byte offset of the lane's cell in row r (fewer than 2^28 cells)
   auto qcell = [&](int r) -> unsigned {
     int rr = r;
     if (per_i) { if (rr < 0 || rr >= ni) rr = wrapi(rr, ni); }
     else rr = min(max(rr, 0), ni - 1);
-    return unsigned(rr) * unsigned(nj) + unsigned(cq);
+    return (unsigned(rr) * unsigned(nj) + unsigned(cq)) * 4u;
   };
 
   // The march: pass r (from r0 - 1) forms the gradient sums of row r + 1, the j-faces of row
@@ -259,116 +338,120 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const float* p = a.q + v * ncell;
-      qa[v] = p[k0];
-      qb[v] = p[k1];
-      qc[v] = p[k2];
-      qn[v] = p[k3];
+      qa[v] = at(p, k0);
+      qb[v] = at(p, k1);
+      qc[v] = at(p, k2);
+      qn[v] = at(p, k3);
     }
   }
-  // offset of the i-face between rows r and r + 1
-  float dxi, dyi;
-  {
-    const float* p = recrow(r0 - 3) + S_DXI * 32 + lane;
-    dxi = p[0];
-    dyi = p[32];
-  }
-  float ma[8], mb[8];   // gradient sums of rows r, r + 1
+  // offset {x, y} of the i-face between rows r and r + 1
+  f2 di = pair_at(recrow(r0 - 3) + S_DXI * 32 + 2 * lane);
+  f2 mx[4], my[4];      // gradient sums {of row r, of row r + 1}, x and y
   float dl[4], dr[4];   // jumps over the left and right faces in row r + 1
   float fi[4], fil = 0.f;  // flux through the i-face r (the upper face of row r)
   float fj[4], fjl = 0.f;  // net j-flux of row r
 #pragma unroll
-  for (int v = 0; v < 4; ++v) { fi[v] = fj[v] = 0.f; ma[2 * v] = ma[2 * v + 1] = 0.f; }
+  for (int v = 0; v < 4; ++v) { fi[v] = fj[v] = 0.f; mx[v] = my[v] = pair(0.f, 0.f); }
 
   // gradient sums (lsq/qmetric.ipp) of row r + 1 from rows r, r + 1, r + 2
   auto gradient = [&](const float* s) {
-    const float xj0 = s[S_DXJ * 32 + lane], yj0 = s[(S_DXJ + 1) * 32 + lane];
-    const float xj1 = s[S_DXJ * 32 + lane + 1], yj1 = s[(S_DXJ + 1) * 32 + lane + 1];
-    const float xi1 = s[S_DXI * 32 + lane], yi1 = s[(S_DXI + 1) * 32 + lane];
+    const f2 dj0 = pair_at(s + S_DXJ * 32 + 2 * lane), dj1 = pair_at(s + S_DXJ * 32 + 2 * lane + 2);
+    const f2 di1 = pair_at(s + S_DXI * 32 + 2 * lane);
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const float left = __shfl_up_sync(0xffffffffu, qb[v], 1);
       dl[v] = qb[v] - left;
       dr[v] = __shfl_down_sync(0xffffffffu, dl[v], 1);
       const float a0 = qb[v] - qa[v], a1 = qc[v] - qb[v];
-      mb[2 * v] = fmaf(dr[v], xj1, fmaf(dl[v], xj0, fmaf(a1, xi1, a0 * dxi)));
-      mb[2 * v + 1] = fmaf(dr[v], yj1, fmaf(dl[v], yj0, fmaf(a1, yi1, a0 * dyi)));
+      const f2 m = fma2(pair(dr[v], dr[v]), dj1,
+                        fma2(pair(dl[v], dl[v]), dj0, fma2(pair(a1, a1), di1, mul2(pair(a0, a0), di))));
+      mx[v] = pair(lo(mx[v]), lo(m));
+      my[v] = pair(lo(my[v]), hi(m));
     }
-    dxi = xi1;
-    dyi = yi1;
+    di = di1;
   };
   // flux through the i-face r + 1, between rows r and r + 1
   auto iface = [&](const float* s, int r, Flux5<float>& F) {
-    const float* f = s + S_IF * 32 + lane;
+    const float* f = s + S_IF * 32 + 2 * lane;
     const int face = r + 1;
+    const f2 n = pair_at(f + P_N * 32);
+    const float area = s[(S_IF + P_A) * 32 + lane];
     if (!per_i && (face == 0 || face == ni)) {
-      const bool lo = face == 0;
+      const bool low = face == 0;
       StripEdge e;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) e.q[v] = lo ? qb[v] : qa[v];
-#pragma unroll
-      for (int v = 0; v < 8; ++v) e.m[v] = lo ? mb[v] : ma[v];
-      e.nx = f[P_NX * 32]; e.ny = f[P_NY * 32]; e.A = f[P_A * 32];
-      e.wx = f[(lo ? P_WRX : P_WLX) * 32]; e.wy = f[(lo ? P_WRY : P_WLY) * 32];
-      e.wwx = f[(lo ? P_WLX : P_WRX) * 32]; e.wwy = f[(lo ? P_WLY : P_WRY) * 32];
-      strip_edge_flux<FK, LIM>(a, lo ? 0 : 1, cq, e, want_lam, F);
+      for (int v = 0; v < 4; ++v) {
+        e.q[v] = low ? qb[v] : qa[v];
+        e.m[2 * v] = low ? hi(mx[v]) : lo(mx[v]);
+        e.m[2 * v + 1] = low ? hi(my[v]) : lo(my[v]);
+      }
+      e.nx = lo(n); e.ny = hi(n); e.A = area;
+      const f2 wx = pair_at(f + P_WX * 32), wy = pair_at(f + P_WY * 32);
+      e.wx = low ? hi(wx) : lo(wx); e.wy = low ? hi(wy) : lo(wy);
+      e.wwx = low ? lo(wx) : hi(wx); e.wwy = low ? lo(wy) : hi(wy);
+      strip_edge_flux<FK, LIM>(a, low ? 0 : 1, cq, e, want_lam, F);
       return;
     }
-    float ql[4], qr[4];
+    f2 q[4];  // {left, right}
     {
-      const float cl = f[P_CL * 32], cr = f[P_CR * 32];
-      const float wlx = f[P_WLX * 32], wly = f[P_WLY * 32], sl = f[P_SL * 32];
-      const float wrx = f[P_WRX * 32], wry = f[P_WRY * 32], sr = f[P_SR * 32];
+      const f2 wx = pair_at(f + P_WX * 32), wy = pair_at(f + P_WY * 32), ns = pair_at(f + P_S * 32),
+               c = pair_at(f + P_C * 32);
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        const float dq = qb[v] - qa[v];
-        const float gl = fmaf(-dq, sl, fmaf(ma[2 * v + 1], wly, ma[2 * v] * wlx));
-        const float gr = fmaf(-dq, sr, fmaf(mb[2 * v + 1], wry, mb[2 * v] * wrx));
-        ql[v] = fmaf(cl, strip_limit<LIM>(dq, gl), qa[v]);
-        qr[v] = fmaf(-cr, strip_limit<LIM>(dq, gr), qb[v]);
+        const float d = qb[v] - qa[v];
+        const f2 dq = pair(d, d);
+        const f2 gr = fma2(dq, ns, fma2(my[v], wy, mul2(mx[v], wx)));
+        q[v] = fma2(c, strip_limit2<LIM>(dq, gr), pair(qa[v], qb[v]));
       }
     }
     St<float> l, rr;
-    basis_state2(g, ql, qr, false, l, rr);
-    F = face_flux<float, FK>(g, f[P_NX * 32], f[P_NY * 32], f[P_A * 32], l, rr, want_lam);
+    strip_states(g, q, l, rr);
+    F = face_flux<float, FK>(g, lo(n), hi(n), area, l, rr, want_lam);
   };
   // flux through the lane's left j-face in row r + 1
   auto jface = [&](const float* s, int r, Flux5<float>& F) {
-    const float* f = s + S_JF * 32 + lane;
-    float ql[4], qr[4];
+    const float* f = s + S_JF * 32 + 2 * lane;
+    const f2 n = pair_at(f + P_N * 32);
+    const float area = s[(S_JF + P_A) * 32 + lane];
+    f2 q[4];  // {left, right}
     {
-      // this cell's state at its right face (the next lane's record), handed to the next lane
-      const float cl = f[P_CL * 32 + 1], wlx = f[P_WLX * 32 + 1], wly = f[P_WLY * 32 + 1], sl = f[P_SL * 32 + 1];
-      const float cr = f[P_CR * 32], wrx = f[P_WRX * 32], wry = f[P_WRY * 32], sr = f[P_SR * 32];
+      // this cell's states at its right face, handed to the next lane, and at its left face
+      const f2 wx = pair_at(f + P_WX * 32), wy = pair_at(f + P_WY * 32), ns = pair_at(f + P_S * 32),
+               c = pair_at(f + P_C * 32);
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        const float gl = fmaf(-dr[v], sl, fmaf(mb[2 * v + 1], wly, mb[2 * v] * wlx));
-        const float gr = fmaf(-dl[v], sr, fmaf(mb[2 * v + 1], wry, mb[2 * v] * wrx));
-        const float mine = fmaf(cl, strip_limit<LIM>(dr[v], gl), qb[v]);
-        ql[v] = __shfl_up_sync(0xffffffffu, mine, 1);
-        qr[v] = fmaf(-cr, strip_limit<LIM>(dl[v], gr), qb[v]);
+        const f2 dq = pair(dr[v], dl[v]);
+        const f2 gr = fma2(dq, ns, fma2(pair(hi(my[v]), hi(my[v])), wy, mul2(pair(hi(mx[v]), hi(mx[v])), wx)));
+        const f2 x = fma2(c, strip_limit2<LIM>(dq, gr), pair(qb[v], qb[v]));
+        q[v] = pair(__shfl_up_sync(0xffffffffu, lo(x), 1), hi(x));
       }
     }
     {
       St<float> l, rr;
-      basis_state2(g, ql, qr, false, l, rr);
-      F = face_flux<float, FK>(g, f[P_NX * 32], f[P_NY * 32], f[P_A * 32], l, rr, want_lam);
+      strip_states(g, q, l, rr);
+      F = face_flux<float, FK>(g, lo(n), hi(n), area, l, rr, want_lam);
     }
     if (edge_j) {
       // on side 3 the interior cell is the lane to the left; its state is also this lane's
       // (columns past the mesh repeat the last one)
       StripEdge e;
 #pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const float left = __shfl_up_sync(0xffffffffu, mb[v], 1);
-        e.m[v] = jside == 3 ? left : mb[v];
+      for (int v = 0; v < 4; ++v) {
+        const float x = hi(mx[v]), y = hi(my[v]);
+        const float xl = __shfl_up_sync(0xffffffffu, x, 1), yl = __shfl_up_sync(0xffffffffu, y, 1);
+        e.m[2 * v] = jside == 3 ? xl : x;
+        e.m[2 * v + 1] = jside == 3 ? yl : y;
       }
       if (jside >= 0) {
-        const bool lo = jside == 2;
+        const bool low = jside == 2;
 #pragma unroll
         for (int v = 0; v < 4; ++v) e.q[v] = qb[v];
-        e.nx = f[P_NX * 32]; e.ny = f[P_NY * 32]; e.A = f[P_A * 32];
-        e.wx = f[(lo ? P_WRX : P_WLX) * 32]; e.wy = f[(lo ? P_WRY : P_WLY) * 32];
-        e.wwx = f[(lo ? P_WLX : P_WRX) * 32]; e.wwy = f[(lo ? P_WLY : P_WRY) * 32];
+        e.nx = lo(n); e.ny = hi(n); e.A = area;
+        // the left face's weights: its left side's in the pair of the lane before
+        const float wlx = f[P_WX * 32 - 2], wly = f[P_WY * 32 - 2];
+        const float wrx = f[P_WX * 32 + 1], wry = f[P_WY * 32 + 1];
+        e.wx = low ? wrx : wlx; e.wy = low ? wry : wly;
+        e.wwx = low ? wlx : wrx; e.wwy = low ? wly : wry;
         strip_edge_flux<FK, LIM>(a, jside, r + 1, e, want_lam, F);
       }
       __syncwarp();
@@ -383,7 +466,10 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
       qc[v] = qn[v];
     }
 #pragma unroll
-    for (int v = 0; v < 8; ++v) ma[v] = mb[v];
+    for (int v = 0; v < 4; ++v) {
+      mx[v] = pair(hi(mx[v]), hi(mx[v]));
+      my[v] = pair(hi(my[v]), hi(my[v]));
+    }
   };
 
   const bool sum_in = a.stage > 0;
@@ -397,7 +483,7 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
 #pragma unroll 1
   for (int r = r0 - 1; r < r1; ++r) {
     const float* s = strip_wait(ring, a.info);
-    const unsigned cell = unsigned(max(r, 0)) * unsigned(nj) + unsigned(cq);
+    const unsigned cell = (unsigned(max(r, 0)) * unsigned(nj) + unsigned(cq)) * 4u;
     gradient(s);
     float jn[4], jnl = 0.f;
 #pragma unroll
@@ -415,7 +501,7 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
       const unsigned c3 = qcell(r + 3);
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        qn[v] = (a.q + v * ncell)[c3];
+        qn[v] = at(a.q + v * ncell, c3);
         pq[v] = qa[v];
         ps[v] = 0.f;
       }
@@ -423,12 +509,12 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
     if (update && own && r >= r0) {
       if (a.q0 != a.q) {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) pq[v] = (a.q0 + v * ncell)[cell];
+        for (int v = 0; v < 4; ++v) pq[v] = at(a.q0 + v * ncell, cell);
       }
       if (sum_in) {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) ps[v] = (sums + v * ncell)[cell];
-        if (a.mode == MODE_FUSED_LOCAL) pl = (sums + 4 * ncell)[cell];
+        for (int v = 0; v < 4; ++v) ps[v] = at(sums + v * ncell, cell);
+        if (a.mode == MODE_FUSED_LOCAL) pl = at(sums + 4 * ncell, cell);
       }
     }
     // face-to-cell accumulation (residualCalc.h:199-253 signs)
@@ -453,8 +539,8 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
       if (a.mode == MODE_RES_MAXRATE || a.mode == MODE_RESIDUAL) {
         if (a.res_out) {
 #pragma unroll
-          for (int v = 0; v < 4; ++v) (a.res_out + v * ncell)[cell] = res[v];
-          (a.res_out + 4 * ncell)[cell] = lam;
+          for (int v = 0; v < 4; ++v) at(a.res_out + v * ncell, cell) = res[v];
+          at(a.res_out + 4 * ncell, cell) = lam;
         }
         rate = fmaxf(rate, div_near(lam, vol));
         r2 = fmaf(res[2], res[2], r2);
@@ -467,15 +553,15 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             tot[v] = fmaf(al, res[v], ap * ps[v]);
-            if (a.res_out) (const_cast<float*>(sums) + v * ncell)[cell] = ps[v] + res[v];
+            if (a.res_out) at(const_cast<float*>(sums) + v * ncell, cell) = ps[v] + res[v];
           }
         } else {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             tot[v] = al * res[v];
-            if (a.res_out) (a.res_out + v * ncell)[cell] = res[v];
+            if (a.res_out) at(a.res_out + v * ncell, cell) = res[v];
           }
-          if (a.res_out) (a.res_out + 4 * ncell)[cell] = lam;
+          if (a.res_out) at(a.res_out + 4 * ncell, cell) = lam;
           rate = fmaxf(rate, div_near(lam, vol));
           r2 = fmaf(res[2], res[2], r2);
         }
@@ -490,8 +576,8 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
         float qo[4];
         forward_update(g, pq, tot, fac, qo, false);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) (a.q_out + v * ncell)[cell] = qo[v];
-        flag_nonphysical(a.info, qo, int(cell));
+        for (int v = 0; v < 4; ++v) at(a.q_out + v * ncell, cell) = qo[v];
+        flag_nonphysical(a.info, qo, int(cell / 4u));
       }
     }
     shift();

@@ -20,41 +20,44 @@ __global__ void pack_strips_kernel(const double* __restrict__ fi, const double* 
     auto row_cell = [&](int i) { return per_i ? wrapi(i, ni) : min(max(i, 0), ni - 1); };
     auto row_face = [&](int i) { return per_i ? wrapi(i, ni) : min(max(i, 0), ni); };
     auto in_row = [&](int i, int n) { return per_i || (i >= 0 && i < n); };
-    float* o = out + (size_t(w) * rows + (r + kStripRowsBefore)) * kStripRow + lane;
-    auto put = [&](int f, double v) { o[f * 32] = float(v); };
+    float* o = out + (size_t(w) * rows + (r + kStripRowsBefore)) * kStripRow;
+    auto put = [&](int f, double v) { o[f * 32 + lane] = float(v); };
+    auto put2 = [&](int f, double x, double y) { o[f * 32 + 2 * lane] = float(x); o[f * 32 + 2 * lane + 1] = float(y); };
     {  // the gradient sums of row r + 1
       const size_t f = size_t(row_cell(r + 1)) * (nj + 1) + cf;
       const bool ok = in_c && in_row(r + 1, ni);
-      put(S_DXJ, ok ? fj[F_DXX * nfj + f] : 0.);
-      put(S_DXJ + 1, ok ? fj[F_DXY * nfj + f] : 0.);
+      put2(S_DXJ, ok ? fj[F_DXX * nfj + f] : 0., ok ? fj[F_DXY * nfj + f] : 0.);
       const size_t g = size_t(row_face(r + 2)) * nj + cc;
       const bool oi = in_row(r + 2, ni + 1);
-      put(S_DXI, oi ? fi[F_DXX * nfi + g] : 0.);
-      put(S_DXI + 1, oi ? fi[F_DXY * nfi + g] : 0.);
+      put2(S_DXI, oi ? fi[F_DXX * nfi + g] : 0., oi ? fi[F_DXY * nfi + g] : 0.);
     }
-    // a face: its limiter weights scaled by dl + dr; on a boundary face the interior side's,
-    // with half the (mirrored) distance, and the wall extrapolation weights as they are
-    auto face = [&](int base, const double* rec, size_t nf, size_t f, int side) {
-      const double dl = rec[F_DL * nf + f], dr = rec[F_DR * nf + f], d = dl + dr;
-      put(base + P_NX, rec[F_NX * nf + f]);
-      put(base + P_NY, rec[F_NY * nf + f]);
-      put(base + P_A, rec[F_A * nf + f]);
-      put(base + P_CL, dl / d);
-      put(base + P_CR, dr / d);
-      const double sl = side == 0 ? 1. : d, sr = side == 1 ? 1. : d;  // side 0: low boundary, 1: high
-      put(base + P_WLX, rec[F_WLX * nf + f] * sl);
-      put(base + P_WLY, rec[F_WLY * nf + f] * sl);
-      put(base + P_SL, rec[F_SL * nf + f] * sl);
-      put(base + P_WRX, rec[F_WRX * nf + f] * sr);
-      put(base + P_WRY, rec[F_WRY * nf + f] * sr);
-      put(base + P_SR, rec[F_SR * nf + f] * sr);
+    // A face: the limiter weights of its left side (of face fl) and of its right side (of face fr;
+    // the same for an i-face) scaled by dl + dr; on a boundary face the interior side's, with
+    // half the (mirrored) distance, and the wall extrapolation weights as they are.  side: 0 the
+    // low boundary's face, 1 the high one's, -1 neither.
+    auto face = [&](int base, const double* rec, size_t nf, size_t fl, int side_l, size_t fr, int side_r) {
+      const double dl = rec[F_DL * nf + fl] + rec[F_DR * nf + fl], dr = rec[F_DL * nf + fr] + rec[F_DR * nf + fr];
+      const double sl = side_l == 0 ? 1. : dl, sr = side_r == 1 ? 1. : dr;
+      put2(base + P_WX, rec[F_WLX * nf + fl] * sl, rec[F_WRX * nf + fr] * sr);
+      put2(base + P_WY, rec[F_WLY * nf + fl] * sl, rec[F_WRY * nf + fr] * sr);
+      put2(base + P_S, -(rec[F_SL * nf + fl] * sl), -(rec[F_SR * nf + fr] * sr));
+      put2(base + P_C, rec[F_DL * nf + fl] / dl, -(rec[F_DR * nf + fr] / dr));
+      put2(base + P_N, rec[F_NX * nf + fr], rec[F_NY * nf + fr]);
+      put(base + P_A, rec[F_A * nf + fr]);
     };
     {
       const int i = row_face(r + 1);
-      face(S_IF, fi, nfi, size_t(i) * nj + cc, per_i ? -1 : (i == 0 ? 0 : (i == ni ? 1 : -1)));
+      const size_t f = size_t(i) * nj + cc;
+      const int side = per_i ? -1 : (i == 0 ? 0 : (i == ni ? 1 : -1));
+      face(S_IF, fi, nfi, f, side, f, side);
     }
     put(S_VOL, vol[size_t(row_cell(r)) * nj + cc]);
-    face(S_JF, fj, nfj, size_t(row_cell(r + 1)) * (nj + 1) + cf, per_j ? -1 : (cf == 0 ? 0 : (cf == nj ? 1 : -1)));
+    {
+      const int cr = per_j ? wrapi(c + 1, nj) : min(max(c + 1, 0), nj);  // the cell's right j-face
+      const size_t row = size_t(row_cell(r + 1)) * (nj + 1);
+      auto side = [&](int f) { return per_j ? -1 : (f == 0 ? 0 : (f == nj ? 1 : -1)); };
+      face(S_JF, fj, nfj, row + cr, side(cr), row + cf, side(cf));
+    }
   }
 }
 
