@@ -15,6 +15,7 @@
 //   j-faces    FREC planes of ni*(nj+1) records, face (i,j) between cells (i,j-1),(i,j)
 #pragma once
 
+#include "hc_pair.cuh"
 #include "hc_physics.cuh"
 
 #include <cstdint>
@@ -201,6 +202,7 @@ template <class R> __device__ __forceinline__ void basis_to_cons(const Gas<R>& g
 // conversions between the storage type R and the compute type C of a stage
 template <class To, class From> __device__ __forceinline__ To cvt(From x) { return To(x); }
 template <> __device__ __forceinline__ double cvt<double, df64>(df64 x) { return x.to_double(); }
+template <> __device__ __forceinline__ df64 cvt<df64, double>(double x) { return dd::split(x); }
 template <class C, class R> __device__ __forceinline__ Gas<C> gas_as(const Gas<R>& g) {
   Gas<C> o;
   o.gamma = cvt<C>(g.gamma); o.gm1 = cvt<C>(g.gm1); o.gamma1 = cvt<C>(g.gamma1);
@@ -341,23 +343,23 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
 #pragma unroll
     for (int q = 0; q < 8; ++q) m[q] = C(0);
     if (ok) {
-      // the cell's four faces: (face index, neighbour offset, is pair face)
+      // the cell's four faces: (face index, neighbour offset, two cells on it)
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
         const bool idir = f < 2;
         const int hi = f & 1;
         int fidx;
-        bool pair;
+        bool inner;
         if (idir) {
           const int fi = gi + hi;
-          pair = (fi > 0 && fi < ni) || per_i;
+          inner = (fi > 0 && fi < ni) || per_i;
           fidx = fi * nj + gj;
         } else {
           const int fj = gj + hi;
-          pair = (fj > 0 && fj < nj) || per_j;
+          inner = (fj > 0 && fj < nj) || per_j;
           fidx = gi * (nj + 1) + fj;
         }
-        if (!pair) continue;
+        if (!inner) continue;
         const C* rec = idir ? cfi : cfj;
         const int nf = idir ? nfi : nfj;
         const C dx = rec[size_t(F_DXX) * nf + fidx], dy = rec[size_t(F_DXY) * nf + fidx];
@@ -366,8 +368,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
         for (int v = 0; v < 4; ++v) {
           // (q_right - q_left) of the face
           const C dq = hi ? (Q(v, na, nb) - Q(v, la, lb)) : (Q(v, la, lb) - Q(v, na, nb));
-          m[2 * v] = mad(dq, dx, m[2 * v]);
-          m[2 * v + 1] = mad(dq, dy, m[2 * v + 1]);
+          if constexpr (std::is_same<C, df64>::value) {
+            const df2 s = pair(dq) * pair(dx, dy) + pair(m[2 * v], m[2 * v + 1]);
+            m[2 * v] = hc::lo(s);
+            m[2 * v + 1] = hc::hi(s);
+          } else {
+            m[2 * v] = mad(dq, dx, m[2 * v]);
+            m[2 * v + 1] = mad(dq, dy, m[2 * v + 1]);
+          }
         }
       }
     }
@@ -444,21 +452,46 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
             C ml[8], mr[8];
             mload(la_l, lb_l, ml);
             mload(la, lb, mr);
+            if constexpr (std::is_same<C, df64>::value && !REC) {
+              // Double-float: the two sides as packed pairs (the same operations and bits).  The
+              // kernel is bound by its chains of dependent FP32 operations and their issue (9,017
+              // instructions a warp and cell, issue 46%): a chain that works for both sides costs
+              // half the instructions of two (two steps of 512 x 1024: 2.09 -> 1.83 ms)
+              const df2 wx = pair(wlx, wrx), wy = pair(wly, wry), sp = pair(sl, sr), d = pair(dl, -dr);
+              df2 q[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const C dq = qr[v] - ql[v];
-              const C gc = dq * idlr;
-              const C gl = (ml[2 * v] * wlx + ml[2 * v + 1] * wly) - dq * sl;
-              const C gr = (mr[2 * v] * wrx + mr[2 * v + 1] * wry) - dq * sr;
-              qL[v] = ql[v] + dl * limit<C>(lim, gc, gl);
-              qR[v] = qr[v] - dr * limit<C>(lim, gc, gr);
-              if constexpr (REC) {
-                sg |= ((unsigned long long)limit_piece<C>(lim, gc, gl) << (4 * v)) |
-                      ((unsigned long long)limit_piece<C>(lim, gc, gr) << (16 + 4 * v));
-                if (a.arg_i) {
-                  double* ag = idir ? a.arg_i + size_t(16) * fidx : a.arg_j + size_t(16) * fidx;
-                  ag[2 * v] = cvt<double>(gc); ag[2 * v + 1] = cvt<double>(gl);
-                  ag[8 + 2 * v] = cvt<double>(gc); ag[9 + 2 * v] = cvt<double>(gr);
+              for (int v = 0; v < 4; ++v) {
+                const C dq = qr[v] - ql[v];
+                const df2 b = (pair(ml[2 * v], mr[2 * v]) * wx + pair(ml[2 * v + 1], mr[2 * v + 1]) * wy) -
+                              pair(dq) * sp;
+                q[v] = pair(ql[v], qr[v]) + d * limit2(lim, dq * idlr, b);
+              }
+              St<C> sL, sR;
+              if (!cons) {
+                prim_states(g, q, sL, sR);
+              } else {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) { qL[v] = hc::lo(q[v]); qR[v] = hc::hi(q[v]); }
+                basis_state2(g, qL, qR, true, sL, sR);
+              }
+              F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
+            } else {
+#pragma unroll
+              for (int v = 0; v < 4; ++v) {
+                const C dq = qr[v] - ql[v];
+                const C gc = dq * idlr;
+                const C gl = (ml[2 * v] * wlx + ml[2 * v + 1] * wly) - dq * sl;
+                const C gr = (mr[2 * v] * wrx + mr[2 * v + 1] * wry) - dq * sr;
+                qL[v] = ql[v] + dl * limit<C>(lim, gc, gl);
+                qR[v] = qr[v] - dr * limit<C>(lim, gc, gr);
+                if constexpr (REC) {
+                  sg |= ((unsigned long long)limit_piece<C>(lim, gc, gl) << (4 * v)) |
+                        ((unsigned long long)limit_piece<C>(lim, gc, gr) << (16 + 4 * v));
+                  if (a.arg_i) {
+                    double* ag = idir ? a.arg_i + size_t(16) * fidx : a.arg_j + size_t(16) * fidx;
+                    ag[2 * v] = cvt<double>(gc); ag[2 * v + 1] = cvt<double>(gl);
+                    ag[8 + 2 * v] = cvt<double>(gc); ag[9 + 2 * v] = cvt<double>(gr);
+                  }
                 }
               }
             }
@@ -468,7 +501,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
             basis_state2(g, qL, qR, cons, sL, sR);
             F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
             sg |= (unsigned long long)flux_bits<C, FK>(g, nx, ny, sL, sR) << SIG_FLUX_SHIFT;
-          } else {
+          } else if constexpr (!std::is_same<C, df64>::value) {
             St<C> sL, sR;
             basis_state2(g, qL, qR, cons, sL, sR);
             F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
@@ -679,8 +712,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
 
 // Resident CTAs per SM the stage kernel is compiled for (measured on the 512x1024
 // O-grid, 256-thread tiles): FP64 2 (its 122 registers; a looser bound lets the
-// compiler take more and costs 13%), double-float 3 and FP32 5 (latency-bound
-// kernels: the extra warps outweigh the few spilled registers, 10-12% faster).
+// compiler take more and costs 13%), double-float 3 (latency-bound: the extra warps
+// outweigh the few spilled registers; two steps 1.62 ms, with 2 CTAs 10% more, with 4
+// 1.72 ms) and FP32, where the strip kernel does not take it, 5.
 template <class R, class C, int NT> struct StageResidency {
   static constexpr int value = std::is_same<R, float>::value ? 1280 / NT
                                : (std::is_same<C, R>::value ? 512 / NT : 768 / NT);

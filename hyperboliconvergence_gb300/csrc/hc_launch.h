@@ -135,11 +135,12 @@ inline void tile_dims(int tile, int* ti, int* tj) {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,                    \
                                          int(StageSmem<TI, TJ, R>::bytes));                              \
     if (e != cudaSuccess) return e;                                                                      \
-    if (std::is_same<R, double>::value && TI == 8 && TJ == 32) {                                          \
-      e = cudaFuncSetAttribute(stage_kernel<8, 32, double, FK, df64>,                                    \
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,                              \
-                               int(StageSmem<8, 32, df64>::bytes));                                      \
-      if (e != cudaSuccess) return e;                                                                    \
+    if (std::is_same<R, double>::value && TI == 8 && TJ == 32) {                                         \
+      for (auto kern : {stage_kernel<8, 32, double, FK, df64>, stage_kernel<8, 32, double, FK, df64, 256, LIM_VANALBADA>,\
+                        stage_kernel<8, 32, double, FK, df64, 256, LIM_VANLEER>}) {                      \
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(StageSmem<8, 32, df64>::bytes));\
+        if (e != cudaSuccess) return e;                                                                  \
+      }                                                                                                  \
     }                                                                                                    \
     return cudaFuncSetAttribute(batch_stage_kernel<TI, TJ, R, FK>,                                       \
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,                             \
@@ -256,10 +257,14 @@ inline void tile_dims(int tile, int* ti, int* tj) {
   }                                                                                                      \
   template <class R> static cudaError_t dispatch(const StageArgs<R>& a, int tile, cudaStream_t s) {     \
     if (std::is_same<R, double>::value && a.fic) {                                                       \
-      /* double-float compute type, 8x32 tiles */                                                        \
+      /* Double-float compute type, 8x32 tiles.  The two limiters with a packed form are compile-time */ \
+      /* constants: the selection among ten, four variables a face, keeps their code from overlapping */ \
+      /* (512 x 1024, van Albada, a step: 0.91 ms chosen at run time, 0.81 so) */                        \
       const dim3 grid((a.nj + 31) / 32, (a.ni + 7) / 8);                                                 \
-      return launch_chained(stage_kernel<8, 32, double, FK, df64>, grid, 256,                           \
-                            StageSmem<8, 32, df64>::bytes, s, a.chained != 0,                            \
+      const auto kern = a.limiter == LIM_VANALBADA ? stage_kernel<8, 32, double, FK, df64, 256, LIM_VANALBADA>\
+                        : a.limiter == LIM_VANLEER ? stage_kernel<8, 32, double, FK, df64, 256, LIM_VANLEER>\
+                                                   : stage_kernel<8, 32, double, FK, df64>;              \
+      return launch_chained(kern, grid, 256, StageSmem<8, 32, df64>::bytes, s, a.chained != 0,           \
                             *reinterpret_cast<const StageArgs<double>*>(&a));                            \
     }                                                                                                    \
     if constexpr (std::is_same<R, float>::value) {                                                       \

@@ -38,6 +38,7 @@
 #pragma once
 
 #include "hc_kernels.cuh"
+#include "hc_pair.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -106,39 +107,6 @@ struct StripArgs {
   int strips, runs;  // strips of the mesh, runs of rows
 };
 
-// ---- pairs of FP32 values: one instruction for two operations (FFMA2 and its kin run at the
-// rate of two FP32 instructions but take one issue slot, which is what bounds the kernel)
-struct f2 { unsigned long long v; };
-__device__ __forceinline__ f2 pair(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float lo(f2 a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
-  return x;
-}
-__device__ __forceinline__ float hi(f2 a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
-  return y;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
 // Value at a byte offset of 32 bits from a plane's base (the same in every lane, so that one
 // address register serves all planes).
 __device__ __forceinline__ float at(const float* plane, unsigned off) {
