@@ -466,15 +466,15 @@ __device__ __forceinline__ void stage_tile(const StageArgs<R>& a, int bi, int bj
                               pair(dq) * sp;
                 q[v] = pair(ql[v], qr[v]) + d * limit2(lim, dq * idlr, b);
               }
-              St<C> sL, sR;
               if (!cons) {
-                prim_states(g, q, sL, sR);
+                F = face_flux_pairs<FK>(g, nx, ny, A, prim_states(g, q), want_lam);
               } else {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) { qL[v] = hc::lo(q[v]); qR[v] = hc::hi(q[v]); }
+                St<C> sL, sR;
                 basis_state2(g, qL, qR, true, sL, sR);
+                F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
               }
-              F = face_flux<C, FK>(g, nx, ny, A, sL, sR, want_lam);
             } else {
 #pragma unroll
               for (int v = 0; v < 4; ++v) {

@@ -13,7 +13,7 @@ using namespace hc;
 __device__ bool same(float a, float b) { return a == b || (a != a && b != b); }
 __device__ bool same(df64 a, df64 b) { return same(a.hi, b.hi) && same(a.lo, b.lo); }
 
-enum { ADD, SUB, MUL, DIV, RCP, ALBADA, LEER, MINMOD, STATE, SPLIT, OPS };
+enum { ADD, SUB, MUL, DIV, RCP, ALBADA, LEER, MINMOD, STATE, SPLIT, ROE, OPS };
 
 __global__ void check(const double* x, int n, int* bad) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -35,11 +35,27 @@ __global__ void check(const double* x, int n, int* bad) {
   Gas<df64> g{};
   g.gamma = df64(1.4); g.gamma1 = df64(2.5);
   const df2 s[4] = {p, q, pair(fabs(c), fabs(a)), pair(fabs(d), fabs(b))};
-  St<df64> l, r;
-  prim_states(g, s, l, r);
+  const StPair sp = prim_states(g, s);
+  const St<df64> l = left_state(sp), r = right_state(sp);
   const St<df64> l0 = prim_state_ir(g, a, c, fabs(c), fabs(d), dd::rcp(fabs(c)));
   const St<df64> r0 = prim_state_ir(g, b, d, fabs(a), fabs(b), dd::rcp(fabs(a)));
   if (!same(l.h, l0.h) || !same(r.h, r0.h) || !same(l.a2, l0.a2) || !same(r.u2, r0.u2)) atomicAdd(&bad[STATE], 1);
+  // a flow: velocities of some units about a density and a pressure near 1, so that the averaged
+  // sound speed is real; sub-, trans- and supersonic faces
+  g.gm1 = df64(0.4);
+  const df64 sc(float(1.0 / 1024.0), 0.f);
+  const df2 t[4] = {p * pair(sc), q * pair(sc), pair(df64(1.0)) + pair(fabs(a), fabs(c)) * pair(sc),
+                    pair(df64(1.0)) + pair(fabs(b), fabs(d)) * pair(sc)};
+  const StPair f = prim_states(g, t);
+  const df64 nx = df64(0.6), ny = df64(-0.8), A = df64(1.75);
+  for (int want = 0; want < 2; ++want) {
+    const Flux5<df64> m = roe_flux_pairs<false>(g, nx, ny, A, f, want), w = roe_flux_pairs<true>(g, nx, ny, A, f, want);
+    const Flux5<df64> m0 = roe_flux<df64, false>(g, nx, ny, A, left_state(f), right_state(f), want);
+    const Flux5<df64> w0 = roe_flux<df64, true>(g, nx, ny, A, left_state(f), right_state(f), want);
+    bool ok = same(m.lam, m0.lam) && same(w.lam, w0.lam);
+    for (int v = 0; v < 4; ++v) ok = ok && same(m.f[v], m0.f[v]) && same(w.f[v], w0.f[v]) && m.f[v].hi == m.f[v].hi;
+    if (!ok) atomicAdd(&bad[ROE], 1);
+  }
   if (!same(dd::split(at(0)), df64(at(0)))) atomicAdd(&bad[SPLIT], 1);
 }
 
@@ -71,7 +87,7 @@ int main() {
   cudaMemcpy(d, wide.data(), wide.size() * 8, cudaMemcpyHostToDevice);
   check<<<unsigned((wide.size() + 255) / 256), 256>>>(d, int(wide.size()), b + OPS);
   if (cudaMemcpy(bad, b, sizeof(bad), cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
-  static const char* names[OPS] = {"add", "sub", "mul", "div", "rcp", "vanalbada", "vanleer", "minmod", "state", "split"};
+  static const char* names[OPS] = {"add", "sub", "mul", "div", "rcp", "vanalbada", "vanleer", "minmod", "state", "split", "roe"};
   for (int o = 0; o < OPS; ++o) std::printf("%s %d\n", names[o], bad[0][o]);
   std::printf("split_wide %d\n", bad[1][SPLIT]);
   return 0;

@@ -7,7 +7,7 @@ import subprocess
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-OPS = ("add", "sub", "mul", "div", "rcp", "vanalbada", "vanleer", "minmod", "state", "split", "split_wide")
+OPS = ("add", "sub", "mul", "div", "rcp", "vanalbada", "vanleer", "minmod", "state", "split", "split_wide", "roe")
 
 
 @pytest.fixture(scope="module")
