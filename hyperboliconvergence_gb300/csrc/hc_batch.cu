@@ -127,8 +127,7 @@ template <class R> int persistent_step(hc_batch* b) {
         HC_CUDA(launch_scalar_batch_update0<R>(a, b->sched.tile, grid, b->cfg.cfl, R(tab.alpha[0][0]),
                                                R(tab.beta[0]), b->stream));
       else
-        HC_CUDA(launch_batch_update0<R>(a, b->sched.tile, grid, b->cfg.cfl, R(tab.alpha[0][0]), R(tab.beta[0]),
-                                        b->stream));
+        HC_CUDA(launch_batch_update0<R>(a, b->sched.tile, b->cfg.cfl, R(tab.alpha[0][0]), R(tab.beta[0]), b->stream));
       b->launches += 2;
     } else {
       a.mode = global ? MODE_FUSED_GLOBAL : MODE_FUSED_LOCAL;

@@ -62,8 +62,13 @@ struct hc_batch {
 
 namespace hc {
 
-template <class R> cudaError_t launch_batch_update0(const BatchArgs<R>& b, int tile, int grid, double cfl,
-                                                    R alpha00, R beta0, cudaStream_t s) {
+// One block per work item: the update has no shared memory to keep, and each item begins with a
+// chain of dependent loads (the list, the instance, its timestep) that a persistent grid of four
+// blocks per SM waits out one after the other.  24 uneven meshes, 2.27 M cells: 85 us of the
+// stage kernel's grid and a quotient per warp, 27 us now (118 MB: 17 us at the copy rate).
+template <class R> cudaError_t launch_batch_update0(const BatchArgs<R>& b, int tile, double cfl, R alpha00, R beta0,
+                                                    cudaStream_t s) {
+  const unsigned grid = unsigned(b.nwork);
   if (tile == HC_TILE_4x32) batch_update0_kernel<4, 32, R><<<grid, 128, 0, s>>>(b, cfl, alpha00, beta0);
   else if (tile == HC_TILE_16x16) batch_update0_kernel<16, 16, R><<<grid, 256, 0, s>>>(b, cfl, alpha00, beta0);
   else batch_update0_kernel<8, 32, R><<<grid, 256, 0, s>>>(b, cfl, alpha00, beta0);

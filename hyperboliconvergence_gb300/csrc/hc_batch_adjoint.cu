@@ -120,7 +120,7 @@ template <class R> int forward_step(BAdj<R>& A, int step, bool rec, int nstages 
         HC_CUDA(launch_scalar_batch_update0<R>(a, tile, grid, b->cfg.cfl, R(A.tab.alpha[0][0]), R(A.tab.beta[0]),
                                                A.s()));
       else
-        HC_CUDA(launch_batch_update0<R>(a, tile, grid, b->cfg.cfl, R(A.tab.alpha[0][0]), R(A.tab.beta[0]), A.s()));
+        HC_CUDA(launch_batch_update0<R>(a, tile, b->cfg.cfl, R(A.tab.alpha[0][0]), R(A.tab.beta[0]), A.s()));
       A.launches += 2;
     } else {
       a.mode = MODE_FUSED_GLOBAL;

@@ -894,26 +894,35 @@ __global__ void __launch_bounds__(TI * TJ, (BatchResidency<R, TI * TJ>::value))
   }
 }
 
-// Stage-0 update of the batch with each instance's own global dt.
+// Stage-0 update of the batch with each instance's own global dt.  One thread of a block forms the
+// timestep: its FP64 quotient takes the FP64 pipe some hundred cycles a warp, for 2.27 M cells
+// 28 us if every warp did.
 template <int TI, int TJ, class R>
 __global__ void __launch_bounds__(TI * TJ) batch_update0_kernel(const BatchArgs<R> b, double cfl, R alpha00, R beta0) {
+  __shared__ R dt_all;
   for (int w = blockIdx.x; w < b.nwork; w += gridDim.x) {
     const int packed = b.order[w];
     const int k = packed >> 16, t = packed & 0xffff;
     const BatchInst& in = b.inst[k];
     StepInfo* info = b.info + k;
-    const R dt = global_dt<R>(info, cfl);
-    if (t == 0 && threadIdx.x == 0) {
-      info->dt = double(dt);
-      info->t += double(dt);
+    if (threadIdx.x == 0) {
+      const R dt = global_dt<R>(info, cfl);
+      dt_all = dt;
+      if (t == 0) {
+        info->dt = double(dt);
+        info->t += double(dt);
+      }
     }
+    __syncthreads();
     const int bi = t / in.tiles_j, bj = t % in.tiles_j;
     const int gi = bi * TI + int(threadIdx.x) / TJ, gj = bj * TJ + int(threadIdx.x) % TJ;
-    if (gi >= in.ni || gj >= in.nj) continue;
-    const size_t ncell = size_t(in.ni) * in.nj;
-    const size_t c = size_t(gi) * in.nj + gj;
-    update0_cell(c, ncell, b.gas, b.q0 + 4 * in.cell, b.res_out + 5 * in.cell, b.vol + in.cell, alpha00,
-                 beta0 * dt, info, b.q_out + 4 * in.cell, b.basis != 0);
+    if (gi < in.ni && gj < in.nj) {
+      const size_t ncell = size_t(in.ni) * in.nj;
+      const size_t c = size_t(gi) * in.nj + gj;
+      update0_cell(c, ncell, b.gas, b.q0 + 4 * in.cell, b.res_out + 5 * in.cell, b.vol + in.cell, alpha00,
+                   beta0 * dt_all, info, b.q_out + 4 * in.cell, b.basis != 0);
+    }
+    __syncthreads();  // dt_all is read before the next item's is written
   }
 }
 
