@@ -768,13 +768,19 @@ __global__ void update0_kernel(int ni, int nj, Gas<R> g, const R* __restrict__ q
                                R* __restrict__ q_out, int advance_time, int basis, double dual_b0dt) {
   const size_t ncell = size_t(ni) * nj;
   chain_wait<std::is_same<R, float>::value>();
-  // dual time: the pseudo step dtau / (1 + b0 dtau / dt) (timestepping/dualTime.ipp:65-66)
-  const R dt = dual_b0dt > 0.0 ? R(dual_step(double(global_dt<R>(info, cfl)), dual_b0dt)) : global_dt<R>(info, cfl);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    info->dt = double(dt);
-    if (advance_time) info->t += double(dt);
+  // one thread of a block forms the timestep (see batch_update0_kernel)
+  __shared__ R dt_all;
+  if (threadIdx.x == 0) {
+    // dual time: the pseudo step dtau / (1 + b0 dtau / dt) (timestepping/dualTime.ipp:65-66)
+    const R dt = dual_b0dt > 0.0 ? R(dual_step(double(global_dt<R>(info, cfl)), dual_b0dt)) : global_dt<R>(info, cfl);
+    dt_all = dt;
+    if (blockIdx.x == 0) {
+      info->dt = double(dt);
+      if (advance_time) info->t += double(dt);
+    }
   }
-  const R dts = beta0 * dt;
+  __syncthreads();
+  const R dts = beta0 * dt_all;
   for (size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x; c < ncell; c += size_t(gridDim.x) * blockDim.x)
     update0_cell(c, ncell, g, q0, res0, vol, alpha00, dts, info, q_out, basis != 0);
 }
