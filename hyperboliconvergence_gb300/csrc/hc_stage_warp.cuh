@@ -27,7 +27,7 @@
 // The tiled kernel before the strips (8 x 32 cells, halo and gradient tiles in shared memory,
 // four block barriers) issued a third more at 45%, waiting on barriers and on the j-face records:
 // 0.174 and 0.100 ms; a batch of 24 uneven quadrant problems, SLAU, 20 steps, uploads and downloads
-// included: 18.8 ms, now 14.7.
+// included: 18.8 ms, now 14.0 (with the update's launch, hc_batch.h).
 // Four blocks of four warps per SM: at most 128 registers, which hold a pass without spills (with
 // the edge faces' code out of line the calls cost 48 bytes of spills and 15% of the time), and
 // 512 x 1024 in runs of 8 rows is one wave of 2,368 warps.
