@@ -245,21 +245,30 @@ __device__ __forceinline__ bool strip_poll(uint64_t* bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
+// Whether the copy of fetch k has landed, waiting for it at most kCopyWaitNs.  The lanes' polls may
+// differ, so the warp goes by their vote: one answer, which every lane acts on together.
+__device__ __forceinline__ bool strip_landed(const StripRing& ring, unsigned k) {
+  constexpr unsigned all = 0xffffffffu;
+  uint64_t* bar = &ring.bar[k % kStripSlots];
+  const unsigned parity = (k / kStripSlots) & 1u;
+  if (__all_sync(all, strip_poll(bar, parity))) return true;
+  const unsigned long long t0 = globaltimer_ns();
+  for (;;) {
+    const bool late = __any_sync(all, globaltimer_ns() - t0 > kCopyWaitNs);
+    if (__all_sync(all, strip_poll(bar, parity))) return true;
+    if (late) return false;
+  }
+}
 // wait for the next fetched row (at most kCopyWaitNs) and return its slot
 __device__ __forceinline__ const float* strip_wait(StripRing& ring, StepInfo* info) {
-  const unsigned k = ring.read % kStripSlots, parity = (ring.read / kStripSlots) & 1u;
+  const unsigned k = ring.read;
   ring.read += 1;
-  if (ring.staged && !ring.dead && !strip_poll(&ring.bar[k], parity)) {
-    const unsigned long long t0 = globaltimer_ns();
-    bool late = false;
-    while (!late && !strip_poll(&ring.bar[k], parity)) late = globaltimer_ns() - t0 > kCopyWaitNs;
-    if (__any_sync(0xffffffffu, late)) {
-      ring.dead = true;  // no further copies or waits; the rows computed from here are discarded with the step
-      atomicCAS(&info->status, ST_OK, ST_TIMEOUT);
-    }
+  if (ring.staged && !ring.dead && !strip_landed(ring, k)) {
+    ring.dead = true;  // no further copies or waits; the rows computed from here are discarded with the step
+    atomicCAS(&info->status, ST_OK, ST_TIMEOUT);
   }
   __syncwarp();
-  return ring.slot + k * kStripRow;
+  return ring.slot + (k % kStripSlots) * kStripRow;
 }
 
 // One run of rows [r0, r1) of strip w.
