@@ -807,42 +807,29 @@ int hc_set_bcs(hc_ctx* c, const int bc_type[4], const double* const ref[4]) {
   if (int st = check_ctx(c)) return st;
   if (!c->have_mesh) return fail(HC_ERR_ARG, "upload the mesh before the boundary conditions");
   if (!bc_type) return fail(HC_ERR_ARG, "null bc types");
-  if (c->oned) {  // sides 0 (left) and 1 (right); 2 and 3 do not exist
-    for (int s = 0; s < 2; ++s)
-      if (bc_type[s] < HC_BC_PERIODIC || bc_type[s] > HC_BC_WALL) return fail(HC_ERR_ARG, "unknown bc type");
-    if ((bc_type[0] == HC_BC_PERIODIC) != (bc_type[1] == HC_BC_PERIODIC))
-      return fail(HC_ERR_ARG, "periodic sides must come in pairs (0,1)");
-    for (int s = 0; s < 4; ++s) {
-      c->bc[s] = s < 2 ? bc_type[s] : HC_BC_PERIODIC;
-      c->href[s].clear();
-      if (s < 2 && bc_type[s] != HC_BC_PERIODIC && bc_type[s] != HC_BC_WALL) {
-        if (!ref || !ref[s]) return fail(HC_ERR_ARG, "side " + std::to_string(s) + " needs reference values");
-        c->href[s].assign(ref[s], ref[s] + 3);
-      }
-    }
-    c->have_bcs = true;
-    c->geom_dirty = true;
-    return HC_OK;
-  }
-  for (int s = 0; s < 4; ++s) {
+  // every side is checked before anything changes: a refused call leaves the boundaries as they were
+  // (the geometry is kept below where the types are, so half-written ones would go unnoticed)
+  const int nsides = c->oned ? 2 : 4;  // a line has sides 0 (left) and 1 (right)
+  auto needs = [&](int s) { return bc_type[s] != HC_BC_PERIODIC && bc_type[s] != HC_BC_WALL; };
+  for (int s = 0; s < nsides; ++s) {
     if (bc_type[s] < HC_BC_PERIODIC || bc_type[s] > HC_BC_WALL) return fail(HC_ERR_ARG, "unknown bc type");
     if (c->scalar && (bc_type[s] == HC_BC_ENTROPY || bc_type[s] == HC_BC_WALL))
       return fail(HC_ERR_UNSUPPORTED, "the scalar advection law has periodic, fixed and Riemann boundaries");
   }
-  if ((bc_type[0] == HC_BC_PERIODIC) != (bc_type[1] == HC_BC_PERIODIC) ||
-      (bc_type[2] == HC_BC_PERIODIC) != (bc_type[3] == HC_BC_PERIODIC))
-    return fail(HC_ERR_ARG, "periodic sides must come in pairs (0,1) and (2,3)");
-  // the geometry depends on the boundary types alone
-  bool same = c->have_bcs;
-  for (int s = 0; s < 4; ++s) same = same && c->bc[s] == bc_type[s];
+  for (int s = 0; s < nsides; s += 2)
+    if ((bc_type[s] == HC_BC_PERIODIC) != (bc_type[s + 1] == HC_BC_PERIODIC))
+      return fail(HC_ERR_ARG, c->oned ? "periodic sides must come in pairs (0,1)"
+                                      : "periodic sides must come in pairs (0,1) and (2,3)");
+  for (int s = 0; s < nsides; ++s)
+    if (needs(s) && (!ref || !ref[s])) return fail(HC_ERR_ARG, "side " + std::to_string(s) + " needs reference values");
+  // the geometry of a 2D mesh depends on the boundary types alone
+  bool same = c->have_bcs && !c->oned;
   for (int s = 0; s < 4; ++s) {
-    c->bc[s] = bc_type[s];
+    const int t = s < nsides ? bc_type[s] : HC_BC_PERIODIC;
+    same = same && c->bc[s] == t;
+    c->bc[s] = t;
     c->href[s].clear();
-    const bool needs = bc_type[s] != HC_BC_PERIODIC && bc_type[s] != HC_BC_WALL;
-    if (needs) {
-      if (!ref || !ref[s]) return fail(HC_ERR_ARG, "side " + std::to_string(s) + " needs reference values");
-      c->href[s].assign(ref[s], ref[s] + size_t(c->nv) * c->nface(s));
-    }
+    if (s < nsides && needs(s)) c->href[s].assign(ref[s], ref[s] + (c->oned ? 3 : size_t(c->nv) * c->nface(s)));
   }
   c->have_bcs = true;
   if (same) c->gref_dirty = true;
