@@ -262,11 +262,14 @@ __device__ __forceinline__ bool strip_landed(const StripRing& ring, unsigned k) 
 // wait for the next fetched row (at most kCopyWaitNs) and return its slot
 __device__ __forceinline__ const float* strip_wait(StripRing& ring, StepInfo* info) {
   const unsigned k = ring.read;
-  ring.read += 1;
   if (ring.staged && !ring.dead && !strip_landed(ring, k)) {
     ring.dead = true;  // no further copies or waits; the rows computed from here are discarded with the step
     atomicCAS(&info->status, ST_OK, ST_TIMEOUT);
+    // what is still in flight, this row's copy too, lands (each waited for again, bounded) before
+    // anything else may become of the warp's shared memory
+    for (unsigned f = k; f != ring.used; ++f) (void)strip_landed(ring, f);
   }
+  if (!ring.dead) ring.read = k + 1;  // a dead ring stays at the row that failed
   __syncwarp();
   return ring.slot + (k % kStripSlots) * kStripRow;
 }
@@ -558,17 +561,6 @@ __device__ __forceinline__ void strip_run(const StageArgs<float>& a, const float
       }
     }
     shift();
-  }
-  if (!ring.staged || ring.dead) {
-    // after a wait that ran out: the copies still in flight land (bounded again) before the
-    // warp's shared memory is given up
-    if (ring.dead)
-      for (; ring.read < ring.used; ++ring.read) {
-        const unsigned k = ring.read % kStripSlots, parity = (ring.read / kStripSlots) & 1u;
-        const unsigned long long t0 = globaltimer_ns();
-        while (!strip_poll(&ring.bar[k], parity) && globaltimer_ns() - t0 < kCopyWaitNs) {}
-      }
-    __syncwarp();
   }
   // largest lambda/V and the density-residual norm, once per run
   if (a.mode == MODE_RES_MAXRATE || (a.norm_stage0 && a.stage == 0 && a.mode != MODE_RESIDUAL)) {

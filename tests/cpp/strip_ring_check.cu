@@ -56,10 +56,14 @@ int main() {
   int bad = 0;
   for (int t = 0; t < kThreads; ++t) {
     const bool shorted = (t / 32) % 2 == 1;
-    // a warp dies as a whole at the short row, whose rows before were right; the others read all
-    const bool ok = shorted ? lanes[t].dead == 1 && lanes[t].good >= kShort : lanes[t].dead == 0 && lanes[t].good == kRows;
+    // a warp dies as a whole at the short row, whose rows before were right, and stays there, having
+    // waited for what it had fetched; the others read all
+    const bool ok = shorted ? lanes[t].dead == 1 && lanes[t].good >= kShort && lanes[t].read == kShort &&
+                                  lanes[t].used == kShort + kStripSlots
+                            : lanes[t].dead == 0 && lanes[t].good == kRows && lanes[t].read == kRows &&
+                                  lanes[t].used == kRows;
     if (!ok) {
-      std::printf("thread %d: dead %d good %d\n", t, lanes[t].dead, lanes[t].good);
+      std::printf("thread %d: dead %d good %d used %u read %u\n", t, lanes[t].dead, lanes[t].good, lanes[t].used, lanes[t].read);
       ++bad;
     }
   }
