@@ -162,6 +162,7 @@ def _declare_batch(lib):
         "hc_batch_state_download": [p, i, dp],
         "hc_batch_set_schedule": [p, C.POINTER(Schedule)],
         "hc_batch_set_corrections": [p, C.c_uint],
+        "hc_batch_inject_stalled_copy": [p, C.c_int],
         "hc_batch_set_adjoint_tapes": [p, C.c_int],
         "hc_batch_get_schedule": [p, C.POINTER(Schedule)],
         "hc_batch_step_async": [p, i, i],

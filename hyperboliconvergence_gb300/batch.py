@@ -118,6 +118,11 @@ class Batch:
     def kernel_launches(self) -> int:
         return int(self.lib.hc_batch_kernel_launches(self.h))
 
+    def inject_stalled_copy(self, k: int = -1) -> None:
+        """Test hook of the failure detection (hc_batch_inject_stalled_copy): instance k's copies
+        never complete and its bounded waits run out; -1 clears it."""
+        check(self.lib.hc_batch_inject_stalled_copy(self.h, int(k)))
+
     def set_adjoint_tapes(self, ntapes: int = -1) -> None:
         """Stage tapes of the batched adjoint's checkpointing (hc_batch_set_adjoint_tapes):
         -1 one per snapshot and one more, 0 none, k at most k."""

@@ -163,6 +163,7 @@ template <class R> int per_instance_step(hc_batch* b) {
     base.gas = with_fixes(make_gas<R>(b->gamma, b->Rgas, b->minf), b->fixes);
     base.limiter = b->cfg.limiter;
     base.basis = b->cfg.basis;
+    base.stall_copy = b->stall == k + 1;
     base.fi = (const R*)b->fi + (long long)FREC * b->fi_off[k];
     base.fj = (const R*)b->fj + (long long)FREC * b->fj_off[k];
     base.vol = (const R*)b->vol + b->cell_off[k];
@@ -422,6 +423,16 @@ int hc_batch_set_corrections(hc_batch* b, unsigned mask) {
   if (int st = check_b(b)) return st;
   if (mask & ~unsigned(HC_FIX_ALL)) return fail(HC_ERR_ARG, "unknown correction bits");
   b->fixes = mask;
+  // a captured graph holds the old launch arguments
+  if (b->graph_exec) { cudaGraphExecDestroy(b->graph_exec); b->graph_exec = nullptr; }
+  if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
+  return HC_OK;
+}
+
+int hc_batch_inject_stalled_copy(hc_batch* b, int inst) {
+  if (int st = check_b(b)) return st;
+  if (inst < -1 || inst >= b->ninst) return fail(HC_ERR_ARG, "bad instance");
+  b->stall = inst + 1;
   // a captured graph holds the old launch arguments
   if (b->graph_exec) { cudaGraphExecDestroy(b->graph_exec); b->graph_exec = nullptr; }
   if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }

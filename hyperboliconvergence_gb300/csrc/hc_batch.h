@@ -18,6 +18,7 @@ struct hc_batch {
   std::vector<std::vector<double>> href;  // 4 per instance
   double gamma = 1.4, Rgas = 287.058, minf = 1e-4;
   unsigned fixes = 0;  // HC_FIX_* corrections (hc_batch_set_corrections)
+  int stall = 0;       // test hook (hc_batch_inject_stalled_copy): 1 + the instance, or 0
   int adj_tapes = -1;  // adjoint stage tapes (hc_batch_set_adjoint_tapes); -1 auto
   cudaStream_t own = nullptr, stream = nullptr;
   int sms = 152;
@@ -83,6 +84,7 @@ template <class R> BatchArgs<R> batch_args(hc_batch* b) {
   a.gas = with_fixes(make_gas<R>(b->gamma, b->Rgas, b->minf), b->fixes);
   a.limiter = b->cfg.limiter;
   a.basis = b->cfg.basis;
+  a.stall = b->stall;
   a.q0 = (const R*)b->q[0];
   a.fi = (const R*)b->fi; a.fj = (const R*)b->fj; a.vol = (const R*)b->vol;
   a.gref = (const R*)b->gref;

@@ -821,6 +821,7 @@ template <class R> struct BatchArgs {
   R beta, cfl;
   StepInfo* info;          // one per instance
   int basis;               // solution basis: 0 primitive, 1 conserved
+  int stall;               // test hook (hc_batch_inject_stalled_copy): 1 + the instance, or 0
   // FP32 Euler batches: the packed records of the strip kernel (hc_stage_warp.cuh), its work
   // list and rows per run, and its grid
   const float* pk;
@@ -841,7 +842,7 @@ template <class R> __device__ __forceinline__ StageArgs<R> instance_args(const B
   a.dual_src = nullptr;  // batches have no dual time
   a.dual_g0 = R(1);
   a.dual_b0dt = R(0);
-  a.stall_copy = 0;
+  a.stall_copy = b.stall == k + 1;
   a.plain_loads = 0;
   a.chained = 0;
   a.clear_words = 0;

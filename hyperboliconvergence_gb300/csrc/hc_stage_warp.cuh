@@ -623,6 +623,10 @@ __global__ void __launch_bounds__(32 * kStripWarps, 4) batch_strip_kernel(const 
   for (int i = int(blockIdx.x) * kStripWarps + warp; i < b.strip_work; i += int(gridDim.x) * kStripWarps) {
     const int packed = b.strip_order[i];
     const int k = packed >> 16, t = packed & 0xffff;
+    if (ring.dead) {  // a copy of an earlier item never landed: this one cannot be computed either
+      if (lane == 0) atomicCAS(&b.info[k].status, ST_OK, ST_TIMEOUT);
+      continue;
+    }
     if (lane == 0) sa[warp] = instance_args(b, k);
     __syncwarp();
     const StageArgs<float>& a = sa[warp];

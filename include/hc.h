@@ -458,6 +458,9 @@ int hc_batch_state_upload(hc_batch* b, int inst, const double* prim_soa);
 int hc_batch_state_download(hc_batch* b, int inst, double* prim_soa);
 int hc_batch_set_schedule(hc_batch* b, const hc_schedule* s);
 int hc_batch_set_corrections(hc_batch* b, unsigned mask);  /* hc_set_corrections for a batch */
+/* hc_inject_stalled_copy for one instance of an FP32 batch (-1 clears it).  Every instance whose
+ * work a timed-out warp still had to do is marked with it; the others' results stand. */
+int hc_batch_inject_stalled_copy(hc_batch* b, int inst);
 int hc_batch_get_schedule(hc_batch* b, hc_schedule* s);
 /* Enqueue nsteps RK steps of every instance (hc_batch_mode). */
 int hc_batch_step_async(hc_batch* b, int nsteps, int mode);
