@@ -512,12 +512,16 @@ int hc_batch_sync(hc_batch* b, hc_step_stats* stats) {
       stats[k].dt = info[k].dt;
       stats[k].t = info[k].t;
       stats[k].resnorm = std::sqrt(info[k].resnorm2);
-      stats[k].status = info[k].status == ST_OK ? HC_OK : HC_ERR_NONPHYSICAL;
+      stats[k].status = info[k].status == ST_OK        ? HC_OK
+                        : info[k].status == ST_TIMEOUT ? HC_ERR_TIMEOUT
+                                                       : HC_ERR_NONPHYSICAL;
       stats[k].bad_cell = info[k].bad_cell;
       stats[k].kernel_launches = b->launches;
     }
     if (info[k].status != ST_OK && bad < 0) bad = k;
   }
+  if (bad >= 0 && info[bad].status == ST_TIMEOUT)
+    return fail(HC_ERR_TIMEOUT, "instance " + std::to_string(bad) + ": a staged load did not complete in its bounded wait");
   if (bad >= 0)
     return fail(HC_ERR_NONPHYSICAL, "instance " + std::to_string(bad) + ": non-physical state at cell " +
                                         std::to_string(info[bad].bad_cell));

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from hyperboliconvergence_gb300 import cases
-from hyperboliconvergence_gb300._capi import StepStats
+from hyperboliconvergence_gb300._capi import HC_ERR_TIMEOUT, HCError, StepStats
 from hyperboliconvergence_gb300.batch import Batch
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +47,15 @@ def test_stalled_member(mode):
     code, status, states = step(b, mode)
     assert code == 0 and not any(status)
     assert all(np.array_equal(x, y) for x, y in zip(states, good))
+
+
+def test_timeout_is_reported_as_such():
+    b, _ = make()
+    b.inject_stalled_copy(3)
+    code, status, _ = step(b, "per_instance")
+    assert code == HC_ERR_TIMEOUT
+    assert [s for s in status if s] == [HC_ERR_TIMEOUT] and status[3] == HC_ERR_TIMEOUT
+    b.step_async(1, "per_instance")
+    with pytest.raises(HCError) as err:
+        b.sync()
+    assert err.value.code == HC_ERR_TIMEOUT
