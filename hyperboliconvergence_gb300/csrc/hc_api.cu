@@ -931,6 +931,11 @@ int hc_step_async(hc_ctx* c, int nsteps) {
   if (int st = check_ctx(c)) return st;
   if (nsteps < 0) return fail(HC_ERR_ARG, "negative step count");
   if (int st = ensure_ready(c)) return st;
+  if (nsteps == 0) {
+    // no step: the status is cleared, the last step's rate and norm stay (status, bad_cell adjacent)
+    HC_CUDA(cudaMemsetAsync(&c->info->status, 0, 2 * sizeof(int), c->stream));
+    return HC_OK;
+  }
   // clear the device status of earlier calls, and the first step's words
   HC_CUDA(cudaMemsetAsync(&c->info->maxrate, 0, kCallWords, c->stream));
   c->words_clear = true;
