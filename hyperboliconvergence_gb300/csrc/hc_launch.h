@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <type_traits>
 #include <vector>
 
@@ -29,6 +30,8 @@ inline int device_sms() {
   return sms;
 }
 
+constexpr int kGridRows = 65535;  // a grid's second dimension: the rows of tiles of a launch
+
 // Tile of an FP64 stage launch.  The stage takes as long as its busiest SM, whose time is the
 // FP64 instructions of its tiles: an SM starts one per 19 cycles and each of its four
 // sub-partitions one per 64 (measured), whatever the number of active lanes.  So a tile costs
@@ -38,6 +41,7 @@ inline int device_sms() {
 // 16x16 against this rule): 40 x 40 0.263 -> 0.082, 128 x 128 0.260 -> 0.140, 200 x 200 0.394
 // -> 0.291; SLAU 300 x 401 0.845 -> 0.649; 256 x 512 and larger stay on 16x16.
 inline double f64_tile_cost(int ni, int nj, int ti, int tj, int sms) {
+  if ((ni + ti - 1) / ti > kGridRows) return std::numeric_limits<double>::infinity();  // not launchable
   const long long tiles = (long long)((ni + ti - 1) / ti) * ((nj + tj - 1) / tj);
   const double k = double((tiles + sms - 1) / sms);
   auto pass = [k](int items, int instr) {  // warps of one phase, dealt to four sub-partitions
@@ -46,8 +50,7 @@ inline double f64_tile_cost(int ni, int nj, int ti, int tj, int sms) {
   };
   return pass((ti + 1) * tj + ti * (tj + 1), 230) + pass((ti + 2) * (tj + 2), 48) + pass(ti * tj, 60);
 }
-inline int f64_auto_tile(int ni, int nj) {
-  const int sms = device_sms();
+inline int f64_auto_tile(int ni, int nj, int sms = device_sms()) {
   const double c16 = f64_tile_cost(ni, nj, 16, 16, sms), c8 = f64_tile_cost(ni, nj, 8, 8, sms),
                c4 = f64_tile_cost(ni, nj, 4, 8, sms);
   if (c16 <= c8 && c16 <= c4) return TILE_16x16_H;
