@@ -713,6 +713,7 @@ int hc_mesh_upload_1d(hc_ctx* c, int nc, const double* nodes_x) {
     return fail(HC_ERR_UNSUPPORTED, "the 1D path runs in FP64 or FP32 in the primitive basis");
   for (int i = 0; i < nc; ++i)
     if (!(nodes_x[i + 1] > nodes_x[i])) return fail(HC_ERR_ARG, "1D nodes must increase");
+  HC_CUDA(c->fp32 ? prepare_line_run<float>(c->cfg.flux) : prepare_line_run<double>(c->cfg.flux));
   HC_CUDA(cudaStreamSynchronize(c->stream));
   c->drop_adj_tape();
   c->pool.trim();

@@ -13,31 +13,6 @@ template <class R, int FK> static cudaError_t go1(const Stage1DArgs<R>& a, cudaS
   return cudaGetLastError();
 }
 
-// the cluster of a short line: as many blocks as tiles up to eight, then more warps a block
-template <class R, int FK> static cudaError_t go_run(const LineRunArgs<R>& args, cudaStream_t s) {
-  static const cudaError_t prep = cudaFuncSetAttribute(
-      line_run_kernel<R, FK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLineSmem);
-  if (prep != cudaSuccess) return prep;
-  LineRunArgs<R> a = args;
-  a.tiles = (a.nc + kLineCells - 1) / kLineCells;
-  a.warps = (a.tiles + kLineBlocks - 1) / kLineBlocks;
-  const int blocks = (a.tiles + a.warps - 1) / a.warps;
-  // a warp more for the ghost states, unless neither end has one to compute
-  auto plain = [](int bc) { return bc == BC_PERIODIC || bc == BC_WALL; };
-  const int ghost = plain(a.P.bc[0]) && plain(a.P.bc[1]) ? 0 : 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(blocks));
-  cfg.blockDim = dim3(unsigned(32 * (a.warps + ghost)));
-  cfg.dynamicSmemBytes = kLineSmem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = unsigned(blocks);
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, line_run_kernel<R, FK>, a);
-}
 template <class R> static cudaError_t dispatch_run(const LineRunArgs<R>& a, int flux, cudaStream_t s) {
   switch (flux) {
     case FLUX_ROE: return go_run<R, FLUX_ROE>(a, s);
@@ -50,6 +25,20 @@ template <class R> static cudaError_t dispatch_run(const LineRunArgs<R>& a, int 
     default: return go_run<R, FLUX_CENTRAL>(a, s);
   }
 }
+template <class R> cudaError_t prepare_line_run(int flux) {
+  switch (flux) {
+    case FLUX_ROE: return prepare_run<R, FLUX_ROE>();
+    case FLUX_SLAU: return prepare_run<R, FLUX_SLAU>();
+    case FLUX_SLAU_REF: return prepare_run<R, FLUX_SLAU_REF>();
+    case FLUX_AUSMPUP: return prepare_run<R, FLUX_AUSMPUP>();
+    case FLUX_RUSANOV: return prepare_run<R, FLUX_RUSANOV>();
+    case FLUX_ROE_WS: return prepare_run<R, FLUX_ROE_WS>();
+    case FLUX_ROE_FACE: return prepare_run<R, FLUX_ROE_FACE>();
+    default: return prepare_run<R, FLUX_CENTRAL>();
+  }
+}
+template cudaError_t prepare_line_run<double>(int flux);
+template cudaError_t prepare_line_run<float>(int flux);
 template <> cudaError_t launch_line_run<double>(const LineRunArgs<double>& a, int flux, cudaStream_t s) {
   return dispatch_run(a, flux, s);
 }

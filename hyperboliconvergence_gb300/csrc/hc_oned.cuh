@@ -555,7 +555,36 @@ __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const _
   cluster_barrier();  // no block leaves while another may still write to its shared memory
 }
 
+// the run's shared memory, allowed on the device of the calling thread
+template <class R, int FK> cudaError_t prepare_run() {
+  return cudaFuncSetAttribute(line_run_kernel<R, FK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLineSmem);
+}
+// the cluster of a short line: as many blocks as tiles up to eight, then more warps a block
+template <class R, int FK> cudaError_t go_run(const LineRunArgs<R>& args, cudaStream_t s) {
+  LineRunArgs<R> a = args;
+  a.tiles = (a.nc + kLineCells - 1) / kLineCells;
+  a.warps = (a.tiles + kLineBlocks - 1) / kLineBlocks;
+  const int blocks = (a.tiles + a.warps - 1) / a.warps;
+  // a warp more for the ghost states, unless neither end has one to compute
+  auto plain = [](int bc) { return bc == BC_PERIODIC || bc == BC_WALL; };
+  const int ghost = plain(a.P.bc[0]) && plain(a.P.bc[1]) ? 0 : 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(blocks));
+  cfg.blockDim = dim3(unsigned(32 * (a.warps + ghost)));
+  cfg.dynamicSmemBytes = kLineSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = unsigned(blocks);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, line_run_kernel<R, FK>, a);
+}
 template <class R> cudaError_t launch_line_run(const LineRunArgs<R>& a, int flux, cudaStream_t s);
+// the kernel of a flux made ready on the current device (at every mesh upload: a process may use
+// several devices)
+template <class R> cudaError_t prepare_line_run(int flux);
 
 // stage-0 update of the 1D path with the global timestep
 template <class R>
