@@ -7,6 +7,7 @@
 #include "hc_stage_warp.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <limits>
 #include <type_traits>
@@ -20,14 +21,16 @@ namespace hc {
 enum TileShape { TILE_8x32 = 0, TILE_4x32 = 1, TILE_16x16 = 2, TILE_16x16_H = 3, TILE_COUNT = 4, TILE_AUTO = 5,
                  TILE_8x8 = 6, TILE_4x8 = 7 };
 
+// SMs of the calling thread's device (asked for once per device)
 inline int device_sms() {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 152;
-  }();
-  return sms;
+  constexpr int kDevices = 64;
+  static std::atomic<int> sms[kDevices];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 152;
+  if (dev < kDevices && (n = sms[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 152;
+  if (dev < kDevices) sms[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 constexpr int kGridRows = 65535;  // a grid's second dimension: the rows of tiles of a launch
