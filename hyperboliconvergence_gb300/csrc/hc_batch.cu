@@ -73,10 +73,12 @@ int build_worklist(hc_batch* b) {
   HC_CUDA(cudaMemcpyAsync(b->order_d, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   std::vector<int> strips;
   if (b->pk) {
-    b->strip_rows = strip_run_rows(b->ninst, [&](int k) { return b->ni[k]; }, [&](int k) { return b->nj[k]; }, b->sms);
+    // a work item is packed in 16 bits within its instance; a batch with one that has more strips
+    // (a mesh wider than 1.8 million columns) stays on the tile kernel
+    b->strip_rows =
+        strip_run_rows(b->ninst, [&](int k) { return b->ni[k]; }, [&](int k) { return b->nj[k]; }, b->sms, 0xffff);
     for (int k : perm) {
-      const int nt = strip_count(b->nj[k]) * strip_runs(b->ni[k], b->strip_rows);
-      if (nt > 0xffff) return fail(HC_ERR_UNSUPPORTED, "instance has more than 65535 strips");
+      const int nt = b->strip_rows > 0 ? strip_count(b->nj[k]) * strip_runs(b->ni[k], b->strip_rows) : 0;
       for (int t = 0; t < nt; ++t) strips.push_back((k << 16) | t);
     }
     b->strip_work = int(strips.size());

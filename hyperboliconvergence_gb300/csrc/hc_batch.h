@@ -90,7 +90,7 @@ template <class R> BatchArgs<R> batch_args(hc_batch* b) {
   a.gref = (const R*)b->gref;
   a.cfl = R(b->cfg.cfl);
   a.info = b->info;
-  a.pk = b->pk;
+  a.pk = b->strip_work > 0 ? b->pk : nullptr;
   a.strip_order = b->strip_order_d;
   a.strip_work = b->strip_work;
   a.strip_rows = b->strip_rows;

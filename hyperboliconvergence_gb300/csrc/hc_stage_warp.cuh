@@ -75,20 +75,22 @@ __host__ __device__ inline size_t strip_floats(int ni, int nj) {
 // a batch of 24 meshes, 2.27 M cells, with 8 rows (4.2 waves) 0.64, by this rule (2 waves) 0.57;
 // 96 small ones, 0.47 M cells, 0.255 and 0.20.
 inline int strip_runs(int ni, int rows) { return (ni + rows - 1) / rows; }
-template <class NI, class NJ> inline int strip_run_rows(int n, NI ni, NJ nj, int sms) {
+// most: the work items that a mesh may have (0: any number); 0 is returned where a mesh has more
+// whatever the rows.
+template <class NI, class NJ> inline int strip_run_rows(int n, NI ni, NJ nj, int sms, long long most = 0) {
   constexpr int kResident = 16;  // warps per SM
-  int best = 1;
+  int best = 0;
   double cost = 1e300;
   for (int rows = 1; rows <= 64; ++rows) {
     long long items = 0;
     int longest = 0;
-    bool fits = true;  // a work item is packed in 16 bits within its instance
+    bool fits = true;
     for (int k = 0; k < n; ++k) {
       const int runs = strip_runs(ni(k), rows);
       const long long m = (long long)strip_count(nj(k)) * runs;
       items += m;
       longest = std::max(longest, (ni(k) + runs - 1) / runs);
-      fits = fits && (n == 1 || m <= 0xffff);
+      fits = fits && (most == 0 || m <= most);
     }
     const double c = std::ceil(double(items) / (double(sms) * kResident)) * (longest + 1.7);
     if (fits && c < cost) { cost = c; best = rows; }

@@ -1,5 +1,5 @@
-"""The host rule that picks the FP64 tile (tests/cpp/tile_rule_check.cu), over mesh sizes up to the
-launch limits; no GPU."""
+"""The host rules that pick the FP64 tile and the rows of an FP32 strip run
+(tests/cpp/tile_rule_check.cu), over mesh sizes up to the launch limits; no GPU."""
 import os
 import shutil
 import subprocess
@@ -9,7 +9,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def test_fp64_tile_rule(tmp_path):
+def test_launch_rules(tmp_path):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not available")
