@@ -682,7 +682,6 @@ int hc_mesh_upload(hc_ctx* c, int ni, int nj, const double* nodes_xy) {
     HC_CUDA(cudaMalloc(&c->fi, FREC * nfi * sizeof(float)));
     HC_CUDA(cudaMalloc(&c->fj, FREC * nfj * sizeof(float)));
     HC_CUDA(cudaMalloc(&c->vol, n * sizeof(float)));
-    if (!c->scalar) HC_CUDA(cudaMalloc(&c->pk, strip_floats(ni, nj) * sizeof(float)));
     HC_CUDA(cudaMalloc(&c->staging, 5 * n * sizeof(double)));
   } else {
     c->fi = c->fi64; c->fj = c->fj64; c->vol = c->vol64;
@@ -694,6 +693,8 @@ int hc_mesh_upload(hc_ctx* c, int ni, int nj, const double* nodes_xy) {
   for (int k = 0; k < 3; ++k) HC_CUDA(cudaMalloc(&c->q[k], 4 * n * c->rsz));
   for (int k = 0; k < 4; ++k) HC_CUDA(cudaMalloc(&c->res[k], 5 * n * c->rsz));
   for (int s = 0; s < 4; ++s) HC_CUDA(cudaMalloc(&c->gref[s], 4 * size_t(c->nface(s)) * c->rsz));
+  if (c->fp32 && !c->scalar && strips_for(c->cfg.basis, c->cfg.limiter))
+    HC_CUDA(alloc_strips(&c->pk, strip_floats(ni, nj) * sizeof(float), (ni + 7) / 8 > kGridRows));
   HC_CUDA(cudaMemcpyAsync(c->nodes, nodes_xy, nn * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   HC_CUDA(cudaStreamSynchronize(c->stream));
   c->have_mesh = true;

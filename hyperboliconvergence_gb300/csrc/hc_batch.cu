@@ -310,7 +310,7 @@ int hc_batch_create(const hc_config* cfg, int ninst, const int* ni, const int* n
     e = A(&b->fi, FREC * b->nfi * 4);
     if (e == cudaSuccess) e = A(&b->fj, FREC * b->nfj * 4);
     if (e == cudaSuccess) e = A(&b->vol, b->ncell * 4);
-    if (e == cudaSuccess && !scalar) e = A((void**)&b->pk, b->npk * 4);
+    if (e == cudaSuccess && !scalar && strips_for(cfg->basis, cfg->limiter)) e = alloc_strips(&b->pk, b->npk * 4, false);
   } else if (e == cudaSuccess) {
     b->fi = b->fi64; b->fj = b->fj64; b->vol = b->vol64;
   }

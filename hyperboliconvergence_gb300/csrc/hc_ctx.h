@@ -56,7 +56,7 @@ struct hc_ctx {
   void* fic = nullptr;  // face records as double-float (HC_FP64_DF)
   void* fjc = nullptr;
   void* vol = nullptr;
-  float* pk = nullptr;  // FP32 Euler: the face records in the strip kernel's layout
+  float* pk = nullptr;  // FP32 Euler: the face records in the strip kernel's layout, or null (alloc_strips)
   void* q[3] = {nullptr, nullptr, nullptr};
   void* res[4] = {nullptr, nullptr, nullptr, nullptr};
   void* gref[4] = {nullptr, nullptr, nullptr, nullptr};

@@ -109,10 +109,31 @@ inline cudaError_t launch_chained(K* kernel, dim3 grid, unsigned threads, size_t
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// whether the strip kernel takes an FP32 launch of the 8 x 32 tile
-inline bool strips_take(const float* pk, int basis, int limiter) {
-  return pk && basis == 0 && (limiter == LIM_VANALBADA || limiter == LIM_VANLEER || limiter == LIM_MINMOD ||
-                              limiter == LIM_NOLIMIT2 || limiter == LIM_NOLIMIT3);
+// whether the strip kernel takes an FP32 launch of the 8 x 32 tile: the configuration, and with its
+// packed records there
+inline bool strips_for(int basis, int limiter) {
+  return basis == 0 && (limiter == LIM_VANALBADA || limiter == LIM_VANLEER || limiter == LIM_MINMOD ||
+                        limiter == LIM_NOLIMIT2 || limiter == LIM_NOLIMIT3);
+}
+inline bool strips_take(const float* pk, int basis, int limiter) { return pk && strips_for(basis, limiter); }
+// Memory for packed records, after the rest of a mesh's or batch's; null, and the tile kernel takes
+// the launches, where there is none left, or (above 256 MiB) they would take more than a quarter of
+// what is: 123 bytes a cell on a wide mesh, a fifth of all it needs, but 3,456 a row on a narrow
+// one, 1,152 a cell at three columns, which must not cost it the room for its adjoint.  only: the
+// tile kernel cannot take the mesh (more rows of tiles than a grid has), so they must be had.
+inline cudaError_t alloc_strips(float** pk, size_t bytes, bool only) {
+  *pk = nullptr;
+  if (only) return cudaMalloc((void**)pk, bytes);
+  if (bytes > (size_t(256) << 20)) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaError_t e = cudaMemGetInfo(&free_b, &total_b)) return e;
+    if (bytes > free_b / 4) return cudaSuccess;
+  }
+  const cudaError_t e = cudaMalloc((void**)pk, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  (void)cudaGetLastError();
+  *pk = nullptr;
+  return cudaSuccess;
 }
 // the strip kernel's arguments of one mesh
 inline StripArgs strip_args(const StageArgs<float>& a) {
