@@ -48,7 +48,8 @@ constexpr size_t kCallWords = kStepWords + 2 * sizeof(int);
 // the next one starts when the blocks have ended, its launch already prepared: the FP64 kernels
 // do that, whose blocks must spread evenly over idle SMs (128 x 128 vortex 0.139 ms per step
 // without chaining, 0.142 with the early trigger).  No effect on a kernel launched without the
-// attribute.  FP32 steps, ms: 97 x 131 0.041 -> 0.027, 512 x 1024 0.116 -> 0.104.
+// attribute.  A chained kernel takes no __restrict__ pointers: the buffers it reads may still be
+// written when it starts.  FP32 steps, ms: 97 x 131 0.041 -> 0.027, 512 x 1024 0.116 -> 0.104.
 template <bool EARLY> __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   if (EARLY) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -740,9 +741,9 @@ __global__ void __launch_bounds__(TI * TJ) sig_kernel(const StageArgs<R> a) {
 // Stage-0 update of one cell with the global timestep dt = cfl / max(lambda/V)
 // (timestepping/rungeKutta.h:131-154).
 template <class R>
-__device__ __forceinline__ void update0_cell(size_t c, size_t ncell, const Gas<R>& g, const R* __restrict__ q0,
-                                             const R* __restrict__ res0, const R* __restrict__ vol, R alpha00,
-                                             R dts, StepInfo* info, R* __restrict__ q_out, bool cons) {
+__device__ __forceinline__ void update0_cell(size_t c, size_t ncell, const Gas<R>& g, const R* q0,
+                                             const R* res0, const R* vol, R alpha00,
+                                             R dts, StepInfo* info, R* q_out, bool cons) {
   R tot[4], q[4], qn[4];
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
@@ -763,9 +764,9 @@ template <class R> __device__ __forceinline__ R global_dt(const StepInfo* info, 
 __host__ __device__ __forceinline__ double dual_step(double dtau, double b0dt) { return dtau / (1.0 + b0dt * dtau); }
 
 template <class R>
-__global__ void update0_kernel(int ni, int nj, Gas<R> g, const R* __restrict__ q0, const R* __restrict__ res0,
-                               const R* __restrict__ vol, R alpha00, R beta0, double cfl, StepInfo* info,
-                               R* __restrict__ q_out, int advance_time, int basis, double dual_b0dt) {
+__global__ void update0_kernel(int ni, int nj, Gas<R> g, const R* q0, const R* res0,
+                               const R* vol, R alpha00, R beta0, double cfl, StepInfo* info,
+                               R* q_out, int advance_time, int basis, double dual_b0dt) {
   const size_t ncell = size_t(ni) * nj;
   chain_wait<std::is_same<R, float>::value>();
   // one thread of a block forms the timestep (see batch_update0_kernel)
