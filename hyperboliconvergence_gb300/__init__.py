@@ -6,6 +6,6 @@ the SSP Runge-Kutta update, as hand-written sm_103a CUDA behind the C ABI in
 include/hc.h.
 """
 from ._capi import HCError, load
-from .solver import Mesh, Solver
+from .solver import Mesh, Solver, release_idle
 
-__all__ = ["HCError", "Mesh", "Solver", "load"]
+__all__ = ["HCError", "Mesh", "Solver", "load", "release_idle"]

@@ -69,6 +69,7 @@ def _declare(lib):
     sig = {
         "hc_context_create": [C.POINTER(Config), C.POINTER(p)],
         "hc_context_destroy": [p],
+        "hc_release_idle": [],
         "hc_set_stream": [p, v],
         "hc_get_stream": [p, C.POINTER(C.c_void_p)],
         "hc_mesh_upload": [p, i, i, dp],

@@ -214,7 +214,7 @@ template <class AD> int alloc_tapes(AD& A, int ntapes, int snapshots) {
     size_t free_b = 0, total_b = 0;
     HC_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t per = size_t(A.nst) * A.state_values() * sizeof(*A.sq[0]);
-    free_b += A.pool->idle_bytes;
+    free_b += DevicePool::idle_bytes();
     ntapes = int(std::min<size_t>(size_t(snapshots) + 1, free_b / 2 / std::max<size_t>(per, 1)));
   }
   ntapes = std::min(ntapes, A.nsteps);

@@ -197,7 +197,7 @@ template <class R> int run_step_1d_smoothed(hc_ctx* c) {
   const int nst = tab.nst;
   const bool global = c->cfg.dt_mode == HC_DT_GLOBAL;
   const long long n = c->ni;
-  if (!c->smooth_buf) HC_CUDA(cudaMalloc(&c->smooth_buf, 6 * size_t(n) * sizeof(R)));
+  if (!c->smooth_buf) HC_CUDA(device_alloc(&c->smooth_buf, 6 * size_t(n) * sizeof(R)));
   R* wrk = (R*)c->smooth_buf;
   R* tmp = wrk + 3 * n;
   const int ends = c->bc[0] == HC_BC_PERIODIC ? 'p' : 'a';
@@ -418,9 +418,9 @@ int run_signatures(hc_ctx* c, unsigned long long* sig_i, unsigned long long* sig
   const bool args = arg_i && arg_j;
   unsigned long long* d = nullptr;
   double* da = nullptr;
-  HC_CUDA(cudaMalloc(&d, (nfi + nfj) * sizeof(unsigned long long)));
+  HC_CUDA(device_alloc(&d, (nfi + nfj) * sizeof(unsigned long long)));
   struct Free { void* p; ~Free() { if (p) cudaFree(p); } } guard{d};
-  if (args) HC_CUDA(cudaMalloc(&da, 16 * (nfi + nfj) * sizeof(double)));
+  if (args) HC_CUDA(device_alloc(&da, 16 * (nfi + nfj) * sizeof(double)));
   Free guard_a{da};
   HC_CUDA(cudaMemsetAsync(d, 0, (nfi + nfj) * sizeof(unsigned long long), c->stream));
   if (args) HC_CUDA(cudaMemsetAsync(da, 0, 16 * (nfi + nfj) * sizeof(double), c->stream));
@@ -496,7 +496,7 @@ template <class R> int dual_time_run(hc_ctx* c, const hc_dual_time_controls* ctl
       with_fixes(make_gas<R>(c->gamma, c->Rgas, c->minf, c->lref, c->sdt, c->vscale, c->pscale), c->fixes);
   R* buf = nullptr;
   const bool trap = ms.gamma[1] != 0.0;
-  HC_CUDA(cudaMalloc(&buf, (3 * 4 + (trap ? 5 : 0)) * n * sizeof(R)));
+  HC_CUDA(device_alloc(&buf, (3 * 4 + (trap ? 5 : 0)) * n * sizeof(R)));
   struct Reset {
     hc_ctx* c; void* p;
     ~Reset() { c->dual_src = nullptr; c->dual_g0 = 1.0; c->dual_b0dt = 0.0; cudaFree(p); }
@@ -615,7 +615,7 @@ int hc_context_create(const hc_config* cfg, hc_ctx** out) {
     if (c->scalar) e = c->fp32 ? prepare_scalar_stage<float>() : prepare_scalar_stage<double>();
     else e = c->fp32 ? prepare<float>(cfg->flux) : prepare<double>(cfg->flux);
   }
-  if (e == cudaSuccess) e = cudaMalloc(&c->info, sizeof(StepInfo));
+  if (e == cudaSuccess) e = device_alloc(&c->info, sizeof(StepInfo));
   if (e == cudaSuccess) e = cudaMemset(c->info, 0, sizeof(StepInfo));
   if (e != cudaSuccess) {
     if (c->own) cudaStreamDestroy(c->own);
@@ -625,6 +625,11 @@ int hc_context_create(const hc_config* cfg, hc_ctx** out) {
   }
   c->stream = c->own;
   *out = c;
+  return HC_OK;
+}
+
+int hc_release_idle(void) {
+  DevicePool::trim_all();
   return HC_OK;
 }
 
@@ -669,32 +674,35 @@ int hc_mesh_upload(hc_ctx* c, int ni, int nj, const double* nodes_xy) {
   const size_t n = c->ncell();
   const size_t nfi = size_t(ni + 1) * nj, nfj = size_t(ni) * (nj + 1);
   const size_t nn = size_t(ni + 1) * (nj + 1) * 2;
-  HC_CUDA(cudaMalloc(&c->info, sizeof(StepInfo)));
+  HC_CUDA(device_alloc(&c->info, sizeof(StepInfo)));
   HC_CUDA(cudaMemsetAsync(c->info, 0, sizeof(StepInfo), c->stream));
-  HC_CUDA(cudaMalloc(&c->nodes, nn * sizeof(double)));
-  HC_CUDA(cudaMalloc(&c->cx, n * sizeof(double)));
-  HC_CUDA(cudaMalloc(&c->cy, n * sizeof(double)));
-  HC_CUDA(cudaMalloc(&c->xm, 3 * n * sizeof(double)));
-  HC_CUDA(cudaMalloc(&c->vol64, n * sizeof(double)));
-  HC_CUDA(cudaMalloc(&c->fi64, FREC * nfi * sizeof(double)));
-  HC_CUDA(cudaMalloc(&c->fj64, FREC * nfj * sizeof(double)));
+  HC_CUDA(device_alloc(&c->nodes, nn * sizeof(double)));
+  HC_CUDA(device_alloc(&c->cx, n * sizeof(double)));
+  HC_CUDA(device_alloc(&c->cy, n * sizeof(double)));
+  HC_CUDA(device_alloc(&c->xm, 3 * n * sizeof(double)));
+  HC_CUDA(device_alloc(&c->vol64, n * sizeof(double)));
+  HC_CUDA(device_alloc(&c->fi64, FREC * nfi * sizeof(double)));
+  HC_CUDA(device_alloc(&c->fj64, FREC * nfj * sizeof(double)));
   if (c->fp32) {
-    HC_CUDA(cudaMalloc(&c->fi, FREC * nfi * sizeof(float)));
-    HC_CUDA(cudaMalloc(&c->fj, FREC * nfj * sizeof(float)));
-    HC_CUDA(cudaMalloc(&c->vol, n * sizeof(float)));
-    HC_CUDA(cudaMalloc(&c->staging, 5 * n * sizeof(double)));
+    HC_CUDA(device_alloc(&c->fi, FREC * nfi * sizeof(float)));
+    HC_CUDA(device_alloc(&c->fj, FREC * nfj * sizeof(float)));
+    HC_CUDA(device_alloc(&c->vol, n * sizeof(float)));
+    HC_CUDA(device_alloc(&c->staging, 5 * n * sizeof(double)));
   } else {
     c->fi = c->fi64; c->fj = c->fj64; c->vol = c->vol64;
   }
   if (c->df) {
-    HC_CUDA(cudaMalloc(&c->fic, FREC * nfi * sizeof(df64)));
-    HC_CUDA(cudaMalloc(&c->fjc, FREC * nfj * sizeof(df64)));
+    HC_CUDA(device_alloc(&c->fic, FREC * nfi * sizeof(df64)));
+    HC_CUDA(device_alloc(&c->fjc, FREC * nfj * sizeof(df64)));
   }
-  for (int k = 0; k < 3; ++k) HC_CUDA(cudaMalloc(&c->q[k], 4 * n * c->rsz));
-  for (int k = 0; k < 4; ++k) HC_CUDA(cudaMalloc(&c->res[k], 5 * n * c->rsz));
-  for (int s = 0; s < 4; ++s) HC_CUDA(cudaMalloc(&c->gref[s], 4 * size_t(c->nface(s)) * c->rsz));
-  if (c->fp32 && !c->scalar && strips_for(c->cfg.basis, c->cfg.limiter))
-    HC_CUDA(alloc_strips(&c->pk, strip_floats(ni, nj) * sizeof(float), (ni + 7) / 8 > kGridRows));
+  for (int k = 0; k < 3; ++k) HC_CUDA(device_alloc(&c->q[k], 4 * n * c->rsz));
+  for (int k = 0; k < 4; ++k) HC_CUDA(device_alloc(&c->res[k], 5 * n * c->rsz));
+  for (int s = 0; s < 4; ++s) HC_CUDA(device_alloc(&c->gref[s], 4 * size_t(c->nface(s)) * c->rsz));
+  if (c->fp32 && !c->scalar && strips_for(c->cfg.basis, c->cfg.limiter)) {
+    const size_t bytes = strip_floats(ni, nj) * sizeof(float);
+    // (a mesh that the tile kernel cannot take must have them)
+    HC_CUDA((ni + 7) / 8 > kGridRows ? device_alloc(&c->pk, bytes) : alloc_strips(&c->pk, bytes));
+  }
   HC_CUDA(cudaMemcpyAsync(c->nodes, nodes_xy, nn * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   HC_CUDA(cudaStreamSynchronize(c->stream));
   c->have_mesh = true;
@@ -724,20 +732,20 @@ int hc_mesh_upload_1d(hc_ctx* c, int nc, const double* nodes_x) {
   c->ni = nc; c->nj = 1;
   c->hx.assign(nodes_x, nodes_x + nc + 1);
   const size_t n = size_t(nc), nf = size_t(nc) + 1;
-  HC_CUDA(cudaMalloc(&c->info, sizeof(StepInfo)));
+  HC_CUDA(device_alloc(&c->info, sizeof(StepInfo)));
   HC_CUDA(cudaMemsetAsync(c->info, 0, sizeof(StepInfo), c->stream));
-  HC_CUDA(cudaMalloc(&c->vol64, n * sizeof(double)));
-  HC_CUDA(cudaMalloc(&c->fi64, F1REC * nf * sizeof(double)));
+  HC_CUDA(device_alloc(&c->vol64, n * sizeof(double)));
+  HC_CUDA(device_alloc(&c->fi64, F1REC * nf * sizeof(double)));
   if (c->fp32) {
-    HC_CUDA(cudaMalloc(&c->fi, F1REC * nf * sizeof(float)));
-    HC_CUDA(cudaMalloc(&c->vol, n * sizeof(float)));
-    HC_CUDA(cudaMalloc(&c->staging, 4 * n * sizeof(double)));
+    HC_CUDA(device_alloc(&c->fi, F1REC * nf * sizeof(float)));
+    HC_CUDA(device_alloc(&c->vol, n * sizeof(float)));
+    HC_CUDA(device_alloc(&c->staging, 4 * n * sizeof(double)));
   } else {
     c->fi = c->fi64; c->vol = c->vol64;
   }
-  for (int k = 0; k < 3; ++k) HC_CUDA(cudaMalloc(&c->q[k], 3 * n * c->rsz));
-  for (int k = 0; k < 4; ++k) HC_CUDA(cudaMalloc(&c->res[k], 4 * n * c->rsz));
-  for (int s = 0; s < 2; ++s) HC_CUDA(cudaMalloc(&c->gref[s], 3 * c->rsz));
+  for (int k = 0; k < 3; ++k) HC_CUDA(device_alloc(&c->q[k], 3 * n * c->rsz));
+  for (int k = 0; k < 4; ++k) HC_CUDA(device_alloc(&c->res[k], 4 * n * c->rsz));
+  for (int s = 0; s < 2; ++s) HC_CUDA(device_alloc(&c->gref[s], 3 * c->rsz));
   c->have_mesh = true;
   c->have_bcs = false;
   c->have_state = false;

@@ -67,7 +67,7 @@ int build_worklist(hc_batch* b) {
   if (b->nwork > b->nwork_cap) {
     if (b->order_d) cudaFree(b->order_d);
     b->order_d = nullptr;
-    HC_CUDA(cudaMalloc(&b->order_d, order.size() * sizeof(int)));
+    HC_CUDA(device_alloc(&b->order_d, order.size() * sizeof(int)));
     b->nwork_cap = b->nwork;
   }
   HC_CUDA(cudaMemcpyAsync(b->order_d, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
@@ -85,7 +85,7 @@ int build_worklist(hc_batch* b) {
     if (b->strip_work > b->strip_cap) {
       if (b->strip_order_d) cudaFree(b->strip_order_d);
       b->strip_order_d = nullptr;
-      HC_CUDA(cudaMalloc(&b->strip_order_d, strips.size() * sizeof(int)));
+      HC_CUDA(device_alloc(&b->strip_order_d, strips.size() * sizeof(int)));
       b->strip_cap = b->strip_work;
     }
     HC_CUDA(cudaMemcpyAsync(b->strip_order_d, strips.data(), strips.size() * sizeof(int), cudaMemcpyHostToDevice,
@@ -290,7 +290,7 @@ int hc_batch_create(const hc_config* cfg, int ninst, const int* ni, const int* n
       b->ngref += size_t(4) * (s < 2 ? nj[k] : ni[k]);
     }
   }
-  auto A = [&](void** p, size_t bytes) { return cudaMalloc(p, std::max<size_t>(bytes, 16)); };
+  auto A = [&](void** p, size_t bytes) { return device_alloc(p, std::max<size_t>(bytes, 16)); };
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = A((void**)&b->nodes, b->nnode * 8);
   if (e == cudaSuccess) e = A((void**)&b->cx, b->ncell * 8);
@@ -310,7 +310,7 @@ int hc_batch_create(const hc_config* cfg, int ninst, const int* ni, const int* n
     e = A(&b->fi, FREC * b->nfi * 4);
     if (e == cudaSuccess) e = A(&b->fj, FREC * b->nfj * 4);
     if (e == cudaSuccess) e = A(&b->vol, b->ncell * 4);
-    if (e == cudaSuccess && !scalar && strips_for(cfg->basis, cfg->limiter)) e = alloc_strips(&b->pk, b->npk * 4, false);
+    if (e == cudaSuccess && !scalar && strips_for(cfg->basis, cfg->limiter)) e = alloc_strips(&b->pk, b->npk * 4);
   } else if (e == cudaSuccess) {
     b->fi = b->fi64; b->fj = b->fj64; b->vol = b->vol64;
   }
@@ -538,8 +538,8 @@ int hc_batch_autotune(hc_batch* b, int steps, hc_schedule* best) {
   // keep the states and per-instance step info; every trial starts from them
   void* save_q = nullptr;
   StepInfo* save_info = nullptr;
-  HC_CUDA(cudaMalloc(&save_q, 4 * b->ncell * b->rsz));
-  HC_CUDA(cudaMalloc(&save_info, b->ninst * sizeof(StepInfo)));
+  HC_CUDA(device_alloc(&save_q, 4 * b->ncell * b->rsz));
+  HC_CUDA(device_alloc(&save_info, b->ninst * sizeof(StepInfo)));
   HC_CUDA(cudaMemcpyAsync(save_q, b->q[0], 4 * b->ncell * b->rsz, cudaMemcpyDeviceToDevice, b->stream));
   HC_CUDA(cudaMemcpyAsync(save_info, b->info, b->ninst * sizeof(StepInfo), cudaMemcpyDeviceToDevice, b->stream));
   cudaEvent_t e0, e1;

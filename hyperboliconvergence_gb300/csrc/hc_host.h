@@ -4,6 +4,8 @@
 #include "../../include/hc.h"
 #include "hc_launch.h"
 
+#include <algorithm>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -27,45 +29,105 @@ inline int fail(int code, const std::string& msg) {
 // Device blocks an adjoint gives back, kept by its context or batch for the next one: a
 // gradient takes about 40 blocks, and allocating and freeing them took 3 ms of the 24 ms of the
 // 256 x 512 drag gradient and 4 ms of the 12 ms of an eight-instance batch.  At most kKeep bytes
-// wait idle (beyond that, and for larger runs, blocks go back to the driver at once); a new
-// recording frees those it did not take.  Used by one context or batch, on its stream: a
-// block's next user is ordered behind its last one, and changing the stream waits for the old
-// one.
+// wait idle in a process, whatever the number of its contexts (beyond that, and for larger runs,
+// blocks go back to the driver at once); a new recording frees those of its context that it did
+// not take, hc_release_idle and any allocation of the library that fails free everyone's.  A block
+// is used by one context or batch, on its stream: its next user is ordered behind its last one, and
+// changing the stream waits for the old one.  The lists are behind one lock, as contexts may be
+// used from several threads.
 struct DevicePool {
   static constexpr size_t kKeep = size_t(2) << 30;
-  std::vector<std::pair<void*, size_t>> idle;
-  size_t idle_bytes = 0;
-  cudaError_t take(void** p, size_t bytes) {
+  DevicePool() {
+    std::lock_guard<std::mutex> lock(all().m);
+    all().pools.push_back(this);
+  }
+  ~DevicePool() {
+    trim();
+    std::lock_guard<std::mutex> lock(all().m);
+    auto& v = all().pools;
+    v.erase(std::find(v.begin(), v.end(), this));
+  }
+  DevicePool(const DevicePool&) = delete;
+  DevicePool& operator=(const DevicePool&) = delete;
+  cudaError_t take(void** p, size_t bytes);
+  void give(void* p, size_t bytes) {
+    {
+      std::lock_guard<std::mutex> lock(all().m);
+      if (all().bytes + bytes <= kKeep) {
+        idle.push_back({p, bytes});
+        all().bytes += bytes;
+        return;
+      }
+    }
+    cudaFree(p);
+  }
+  void trim() {
+    std::vector<Block> blocks;
+    {
+      std::lock_guard<std::mutex> lock(all().m);
+      drain(blocks);
+    }
+    for (auto& b : blocks) cudaFree(b.first);
+  }
+  // everyone's; whether there was anything to free
+  static bool trim_all() {
+    std::vector<Block> blocks;
+    {
+      std::lock_guard<std::mutex> lock(all().m);
+      for (DevicePool* p : all().pools) p->drain(blocks);
+    }
+    for (auto& b : blocks) cudaFree(b.first);
+    return !blocks.empty();
+  }
+  static size_t idle_bytes() {
+    std::lock_guard<std::mutex> lock(all().m);
+    return all().bytes;
+  }
+
+ private:
+  using Block = std::pair<void*, size_t>;
+  struct All {
+    std::mutex m;
+    std::vector<DevicePool*> pools;
+    size_t bytes = 0;
+  };
+  static All& all() {
+    static All* a = new All;  // outlives every context, also one freed at the process's end
+    return *a;
+  }
+  void drain(std::vector<Block>& out) {
+    for (auto& b : idle) {
+      all().bytes -= b.second;
+      out.push_back(b);
+    }
+    idle.clear();
+  }
+  std::vector<Block> idle;
+};
+
+// device memory; where there is none left, idle blocks are given back first
+template <class T> cudaError_t device_alloc(T** p, size_t bytes) {
+  cudaError_t e = cudaMalloc((void**)p, bytes);
+  if (e == cudaErrorMemoryAllocation && DevicePool::trim_all()) {
+    (void)cudaGetLastError();
+    e = cudaMalloc((void**)p, bytes);
+  }
+  return e;
+}
+inline cudaError_t DevicePool::take(void** p, size_t bytes) {
+  {
+    std::lock_guard<std::mutex> lock(all().m);
     for (size_t k = 0; k < idle.size(); ++k)
       if (idle[k].second == bytes) {
         *p = idle[k].first;
         idle[k] = idle.back();
         idle.pop_back();
-        idle_bytes -= bytes;
+        all().bytes -= bytes;
         return cudaSuccess;
       }
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && !idle.empty()) {
-      (void)cudaGetLastError();
-      trim();
-      e = cudaMalloc(p, bytes);
-    }
-    return e;
   }
-  void give(void* p, size_t bytes) {
-    if (idle_bytes + bytes > kKeep) {
-      cudaFree(p);
-      return;
-    }
-    idle.push_back({p, bytes});
-    idle_bytes += bytes;
-  }
-  void trim() {
-    for (auto& b : idle) cudaFree(b.first);
-    idle.clear();
-    idle_bytes = 0;
-  }
-};
+  return device_alloc(p, bytes);
+}
 
 // RK tables ssp11..ssp34 (ode.h:107-197)
 struct RKTab {

@@ -119,11 +119,9 @@ inline bool strips_take(const float* pk, int basis, int limiter) { return pk && 
 // Memory for packed records, after the rest of a mesh's or batch's; null, and the tile kernel takes
 // the launches, where there is none left, or (above 256 MiB) they would take more than a quarter of
 // what is: 123 bytes a cell on a wide mesh, a fifth of all it needs, but 3,456 a row on a narrow
-// one, 1,152 a cell at three columns, which must not cost it the room for its adjoint.  only: the
-// tile kernel cannot take the mesh (more rows of tiles than a grid has), so they must be had.
-inline cudaError_t alloc_strips(float** pk, size_t bytes, bool only) {
+// one, 1,152 a cell at three columns, which must not cost it the room for its adjoint.
+inline cudaError_t alloc_strips(float** pk, size_t bytes) {
   *pk = nullptr;
-  if (only) return cudaMalloc((void**)pk, bytes);
   if (bytes > (size_t(256) << 20)) {
     size_t free_b = 0, total_b = 0;
     if (cudaError_t e = cudaMemGetInfo(&free_b, &total_b)) return e;

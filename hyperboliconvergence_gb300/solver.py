@@ -85,6 +85,12 @@ class Mesh1D:
         return 1 if side < 2 else 0
 
 
+def release_idle() -> None:
+    """Give the device blocks that gradients keep for the next one (at most 2 GiB in the process)
+    back to the device, for another library's use (hc_release_idle)."""
+    check(_capi.load().hc_release_idle())
+
+
 class Solver:
     """One mesh, its boundary conditions and state, advanced by explicit RK on the GPU."""
 

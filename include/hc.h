@@ -125,6 +125,11 @@ typedef struct {
 /* Context lifetime.  Replaces the integrate() set-up of timestepping/rungeKutta.h:37-95. */
 int hc_context_create(const hc_config* cfg, hc_ctx** out);
 int hc_context_destroy(hc_ctx* ctx);
+/* Gradients keep their device blocks for the next one of the same context or batch, at most 2 GiB in
+ * the whole process.  This call gives the idle ones of every context and batch back to the device
+ * (for another library's use; this one's own allocations do so by themselves when memory runs out).
+ * Not in the reference. */
+int hc_release_idle(void);
 /* Run the context's kernels on this CUDA stream (a cudaStream_t; NULL = the legacy
  * default stream).  A new context runs on a non-blocking stream of its own, which
  * hc_get_stream returns. */
