@@ -205,6 +205,25 @@ inline void tile_dims(int tile, int* ti, int* tj) {
       default: return false;                                                                            \
     }                                                                                                   \
   }                                                                                                     \
+  /* What the strips leave to the FP32 8x32 tile (the conserved basis, dual time, no packed  */        \
+  /* records), with the common limiters compile-time constants: 256 x 512, 20 steps, SLAU +  */        \
+  /* van Leer, conserved 1.37 ms chosen at run time, 1.15 so; dual time 1.58 and 1.36       */         \
+  template <int LIM> static bool go_lim(const StageArgs<float>& a, cudaStream_t s) {                   \
+    const dim3 grid((a.nj + 31) / 32, (a.ni + 7) / 8);                                                 \
+    launch_chained(stage_kernel<8, 32, float, FK, float, 256, LIM>, grid, 256, StageSmem<8, 32, float>::bytes, s, \
+                   a.chained != 0, a);                                                                 \
+    return true;                                                                                       \
+  }                                                                                                    \
+  static bool go_lims(const StageArgs<float>& a, cudaStream_t s) {                                     \
+    switch (a.limiter) {                                                                               \
+      case LIM_VANALBADA: return go_lim<LIM_VANALBADA>(a, s);                                          \
+      case LIM_VANLEER: return go_lim<LIM_VANLEER>(a, s);                                              \
+      case LIM_MINMOD: return go_lim<LIM_MINMOD>(a, s);                                                \
+      case LIM_NOLIMIT2: return go_lim<LIM_NOLIMIT2>(a, s);                                            \
+      case LIM_NOLIMIT3: return go_lim<LIM_NOLIMIT3>(a, s);                                            \
+      default: return false;                                                                           \
+    }                                                                                                  \
+  }                                                                                                    \
   template <int LIM> static bool gob_strip(const BatchArgs<float>& b, cudaStream_t s) {                 \
     batch_strip_kernel<FK, LIM><<<unsigned(b.strip_grid), 32 * kStripWarps, kStripSmem, s>>>(b);        \
     return true;                                                                                        \
@@ -293,7 +312,8 @@ inline void tile_dims(int tile, int* ti, int* tj) {
                             *reinterpret_cast<const StageArgs<double>*>(&a));                            \
     }                                                                                                    \
     if constexpr (std::is_same<R, float>::value) {                                                       \
-      if ((tile == TILE_8x32 || tile < 0 || tile >= TILE_COUNT) && go_strips(a, s)) return cudaGetLastError(); \
+      if ((tile == TILE_8x32 || tile < 0 || tile >= TILE_COUNT) && (go_strips(a, s) || go_lims(a, s)))   \
+        return cudaGetLastError();                                                                       \
     }                                                                                                    \
     if constexpr (std::is_same<R, double>::value) {                                                      \
       if (tile == TILE_AUTO) tile = f64_auto_tile(a.ni, a.nj);                                           \
