@@ -575,6 +575,12 @@ template <class R> int dual_time_run(hc_ctx* c, const hc_dual_time_controls* ctl
   return HC_OK;
 }
 
+// measured on the 512 x 1024 O-grid (Roe, van Albada): FP64 16x16 cells on 128 threads 2.9%
+// faster than on 256 and 4.4% faster than 8x32 (four CTAs per SM instead of two overlap one
+// another's load and barrier phases; the 544 faces fill whole warps), smaller tiles on small
+// meshes (f64_auto_tile); FP32 8x32 (3.6% faster than 16x16)
+static int default_tile(bool fp32) { return fp32 ? TILE_8x32 : TILE_AUTO; }
+
 extern "C" {
 
 const char* hc_last_error_string(void) { return g_last_error.c_str(); }
@@ -604,11 +610,7 @@ int hc_context_create(const hc_config* cfg, hc_ctx** out) {
   c->nv = c->scalar ? 3 : 4;
   c->fp32 = cfg->precision == HC_FP32;
   c->df = cfg->precision == HC_FP64_DF;
-  // measured on the 512 x 1024 O-grid (Roe, van Albada): FP64 16x16 cells on 128 threads
-  // 2.9% faster than on 256 and 4.4% faster than 8x32 (four CTAs per SM instead of two
-  // overlap one another's load and barrier phases; the 544 faces fill whole warps), smaller
-  // tiles on small meshes (f64_auto_tile); FP32 8x32 (3.6% faster than 16x16)
-  c->tile = c->fp32 ? TILE_8x32 : TILE_AUTO;
+  c->tile = default_tile(c->fp32);
   c->rsz = c->fp32 ? sizeof(float) : sizeof(double);
   cudaError_t e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
   if (e == cudaSuccess) {
@@ -808,8 +810,8 @@ int hc_set_adjoint_tapes(hc_ctx* c, int ntapes) {
 
 int hc_set_tile(hc_ctx* c, int tile) {
   if (int st = check_ctx(c)) return st;
-  if (tile < HC_TILE_8x32 || tile > HC_TILE_16x16_H) return fail(HC_ERR_ARG, "unknown tile shape");
-  c->tile = tile;
+  if (tile < HC_TILE_DEFAULT || tile > HC_TILE_16x16_H) return fail(HC_ERR_ARG, "unknown tile shape");
+  c->tile = tile == HC_TILE_DEFAULT ? default_tile(c->fp32) : tile;
   return HC_OK;
 }
 

@@ -136,10 +136,10 @@ class Solver:
         self.bc = list(bc)
         self.set_bcs(bc, ref)
 
-    def set_tile(self, tile: str) -> None:
-        """Cells per CTA tile of the 2D FP64/FP32 stage kernels: "8x32", "4x32" or "16x16"
-        (the results do not depend on it)."""
-        check(self.lib.hc_set_tile(self.h, _capi.TILE[tile]))
+    def set_tile(self, tile: str | None) -> None:
+        """Cells per CTA tile of the 2D FP64/FP32 stage kernels: "8x32", "4x32", "16x16",
+        "16x16/128" or None, a new solver's choice (the results do not depend on it)."""
+        check(self.lib.hc_set_tile(self.h, _capi.TILE_DEFAULT if tile is None else _capi.TILE[tile]))
         self.tile = tile
 
     def set_corrections(self, corrections) -> None:

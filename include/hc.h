@@ -416,8 +416,9 @@ typedef struct hc_batch hc_batch;
 
 typedef enum { HC_BATCH_PERSISTENT = 0, HC_BATCH_PER_INSTANCE = 1 } hc_batch_mode;
 typedef enum { HC_ORDER_NATURAL = 0, HC_ORDER_LARGEST_FIRST = 1 } hc_batch_order;
-/* HC_TILE_16x16_H: 16 x 16 cells run by 128 threads (single-mesh contexts only) */
-typedef enum { HC_TILE_8x32 = 0, HC_TILE_4x32 = 1, HC_TILE_16x16 = 2, HC_TILE_16x16_H = 3 } hc_tile;
+/* HC_TILE_16x16_H: 16 x 16 cells run by 128 threads; HC_TILE_DEFAULT: a new context's choice (both
+ * single-mesh contexts only) */
+typedef enum { HC_TILE_DEFAULT = -1, HC_TILE_8x32 = 0, HC_TILE_4x32 = 1, HC_TILE_16x16 = 2, HC_TILE_16x16_H = 3 } hc_tile;
 
 typedef struct {
   int tile;         /* hc_tile: cells per CTA tile */
@@ -428,8 +429,9 @@ typedef struct {
 
 /* Tile shape (hc_tile) of a single-mesh context's stage kernels: the FP64 and FP32
  * 2D stage, residual and adjoint-recompute launches (the double-float and 1D kernels
- * keep their own).  Defaults: HC_TILE_16x16_H in FP64 (16 x 16 cells, whose 544 faces
- * fill whole warps, on 128 threads: four CTAs per SM), HC_TILE_8x32 in FP32.  Every shape
+ * keep their own).  HC_TILE_DEFAULT, also a new context's: in FP64 by the mesh's size,
+ * HC_TILE_16x16_H (16 x 16 cells, whose 544 faces fill whole warps, on 128 threads: four CTAs per
+ * SM) or, on small meshes, 8 x 8 or 4 x 8 cells; in FP32 HC_TILE_8x32.  Every shape
  * gives the same results. */
 int hc_set_tile(hc_ctx* ctx, int tile);
 
