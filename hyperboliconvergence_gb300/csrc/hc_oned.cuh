@@ -388,6 +388,18 @@ __device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long b
   return (unsigned long long)hi << 32 | lo;
 }
 
+// x / d by d's inverse r, taken once per launch: the product corrected by its remainder, in three
+// FP64 instructions the quotient rounded once (P. W. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990), where the product alone is off by an ulp.  FP32
+// divides, as the launches per stage do.
+__device__ __forceinline__ float line_div(float x, float d, float) { return div_near(x, d); }
+__device__ __forceinline__ double line_div(double x, double d, double r) {
+  const double q = x * r;
+  // (an infinite or NaN quotient stays)
+  if ((f64_bits(q) & 0x7fffffffffffffffLL) >= 0x7ff0000000000000LL) return q;
+  return fma(fma(-q, d, x), r, q);
+}
+
 template <class R, int FK>
 __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const __grid_constant__ LineRunArgs<R> a) {
   __shared__ LineMail<R> mail[kLineWarps];
@@ -474,7 +486,7 @@ __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const _
       R res[3], lam;
       line_residual<R, FK>(a.P, ref, ghost, G, lane, last, q, qx, s == 0, res, lam);
       if (s == 0) {
-        const R rate = own ? (sizeof(R) == 4 ? div_near(lam, G.vol) : lam * ivol) : R(0);
+        const R rate = own ? line_div(lam, G.vol, ivol) : R(0);
         // a NaN or negative rate does not count, as in atomic_max_rate
         const unsigned long long bits =
             rate > R(0) ? (unsigned long long)__double_as_longlong(double(rate)) : 0ull;
@@ -504,9 +516,8 @@ __global__ void __launch_bounds__(32 * (kLineWarps + 1)) line_run_kernel(const _
       }
       // rungeKuttaAccumulation (timestepping/rungeKutta.h:172-197) and the update
       R cn[3];
-      // FP64 multiplies by the inverses taken once; FP32 divides, as the launches per stage do
-      const R fac = sizeof(R) == 4 ? div_near(a.beta[s] * fac0, a.global ? G.vol : lam0)
-                                   : (a.beta[s] * fac0) * (a.global ? ivol : rcp_fast(lam0));
+      const R fac = a.global ? line_div(a.beta[s] * fac0, G.vol, ivol)
+                             : line_div(a.beta[s] * fac0, lam0, rcp_fast(lam0));
 #pragma unroll
       for (int v = 0; v < 3; ++v) {
         const R tot = mad(a.alpha[s][s], res[v], s > 0 ? a.alpha[s][0] * rs[v] : R(0));
