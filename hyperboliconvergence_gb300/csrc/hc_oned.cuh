@@ -373,7 +373,9 @@ template <class R> struct LineMail {
 // FP64 pipe
 constexpr int kLineSmem = 120 * 1024;
 
+// (its aligned form takes the warp's lanes together, whatever branches came before)
 __device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 template <class T> __device__ __forceinline__ T* cluster_ptr(T* p, unsigned block) {
