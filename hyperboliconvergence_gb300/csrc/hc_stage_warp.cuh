@@ -18,16 +18,17 @@
 // -s (dl + dr), dl/(dl + dr) and -dr/(dl + dr): the limiters are homogeneous, and the division
 // by that distance disappears.
 //
-// What bounds it: instruction issue (60% of the issue slots at four warps per scheduler, no pipe
-// above 30%; 834 instructions per warp and row).  So what comes in twos -- a face's left and
+// What bounds it: instruction issue (58% of the issue slots at four warps per scheduler, FMA 30%, no
+// other pipe above 26%; 845 instructions per warp and row).  So what comes in twos -- a face's left and
 // right side, a gradient's x and y -- is computed as packed FP32 pairs, one instruction for two
 // operations, from records that hold the pairs side by side, and the planes are addressed by a
-// 32-bit byte offset that serves all of them: 912 instructions before, 512 x 1024 O-grid, Roe +
-// van Albada: 0.104 -> 0.096 ms per ssp34 step, 301 x 715, AUSM+up + van Leer: 0.062 -> 0.059.
+// 32-bit byte offset that serves all of them: 912 instructions before and 834 with the pairs (the
+// waits' votes and the roots' selections came later), 512 x 1024 O-grid, Roe + van Albada: 0.104 ->
+// 0.096 ms per ssp34 step (0.097 now), 301 x 715, AUSM+up + van Leer: 0.062 -> 0.059.
 // The tiled kernel before the strips (8 x 32 cells, halo and gradient tiles in shared memory,
 // four block barriers) issued a third more at 45%, waiting on barriers and on the j-face records:
 // 0.174 and 0.100 ms; a batch of 24 uneven quadrant problems, SLAU, 20 steps, uploads and downloads
-// included: 18.8 ms, now 14.0 (with the update's launch, hc_batch.h).
+// included: 18.8 ms, now 14.2 (with the update's launch, hc_batch.h).
 // Four blocks of four warps per SM: at most 128 registers, which hold a pass without spills (with
 // the edge faces' code out of line the calls cost 48 bytes of spills and 15% of the time), and
 // 512 x 1024 in runs of 8 rows is one wave of 2,368 warps.

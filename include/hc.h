@@ -162,7 +162,8 @@ int hc_set_low_mach(hc_ctx* ctx, int velocity_scaling, int pressure_scaling, dou
 /* SolutionField::bcTypes and the reference layer of SolutionField::boundary
  * (solutionField/solutionField.h:56-91).  ref[side] holds 4 planes of values in the
  * context's basis (hc_config.basis), one per boundary face (nj faces on sides 0/1, ni
- * on 2/3); NULL for periodic or wall sides. */
+ * on 2/3); NULL for periodic or wall sides.  Every side is checked before one is set: a refused
+ * call leaves the boundaries as they were. */
 int hc_set_bcs(hc_ctx* ctx, const int bc_type[4], const double* const ref[4]);
 
 /* SolutionField::interior, 4 planes in the context's basis: primitive {u, v, rho, p}
@@ -178,7 +179,8 @@ int hc_state_download_device(hc_ctx* ctx, void* prim_soa_device);
  * out: 5 planes -- 4 conserved flux sums and the spectral-radius sum. */
 int hc_residual(hc_ctx* ctx, double* out5);
 
-/* nsteps explicit RK steps: the time loop of integrate() (timestepping/rungeKutta.h:96-164). */
+/* nsteps explicit RK steps: the time loop of integrate() (timestepping/rungeKutta.h:96-164).
+ * 0 steps change nothing; the stats are the last step's. */
 int hc_step(hc_ctx* ctx, int nsteps, hc_step_stats* stats);
 /* The accumulated time t that hc_step_stats reports (the time integrate() accumulates,
  * timestepping/rungeKutta.h:96-164); uploading a mesh sets it to 0.  A run restored from
