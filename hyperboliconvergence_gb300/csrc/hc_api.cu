@@ -233,6 +233,14 @@ template <class R> int run_step_1d_smoothed(hc_ctx* c) {
   return HC_OK;
 }
 
+// A fused stage must not write the state that its other blocks still read: the one stage of a
+// one-stage table with local timesteps goes through a buffer beside it (a copy, not an exchange of
+// the pointers, so that a captured call can be replayed).
+template <class R> R* beside(hc_ctx* c, const R* in, R* out) { return out == in ? (R*)c->q[1] : out; }
+template <class R> cudaError_t bring_back(hc_ctx* c) {
+  return cudaMemcpyAsync(c->q[0], c->q[1], size_t(c->nv) * c->ncell() * sizeof(R), cudaMemcpyDeviceToDevice, c->stream);
+}
+
 // one RK step of the 1D path (the same stage loop as run_step)
 template <class R> int run_step_1d(hc_ctx* c) {
   if (c->smooth_alpha > 0.0) return run_step_1d_smoothed<R>(c);
@@ -262,8 +270,9 @@ template <class R> int run_step_1d(hc_ctx* c) {
       c->launches += 2;
     } else {
       a.mode = global ? MODE_FUSED_GLOBAL : MODE_FUSED_LOCAL;
-      a.q_out = out_of(s);
+      a.q_out = beside(c, a.q, out_of(s));
       HC_CUDA(launch_stage1d<R>(a, c->cfg.flux, c->stream));
+      if (a.q_out != out_of(s)) HC_CUDA(bring_back<R>(c));
       c->launches += 1;
     }
   }
@@ -366,8 +375,9 @@ template <class R> int run_step(hc_ctx* c, bool first = false, bool last = true)
       c->launches += 2;
     } else {
       a.mode = global ? MODE_FUSED_GLOBAL : MODE_FUSED_LOCAL;
-      a.q_out = out_of(s);
+      a.q_out = beside(c, a.q, out_of(s));
       HC_CUDA(fn(a, c->tile, c->stream));
+      if (a.q_out != out_of(s)) HC_CUDA(bring_back<R>(c));
       c->launches += 1;
     }
   }

@@ -133,8 +133,11 @@ template <class R> int persistent_step(hc_batch* b) {
       b->launches += 2;
     } else {
       a.mode = global ? MODE_FUSED_GLOBAL : MODE_FUSED_LOCAL;
-      a.q_out = out_of(s);
+      // (one stage, local timesteps: not onto the state that other blocks still read)
+      a.q_out = out_of(s) == a.q ? (R*)b->q[1] : out_of(s);
       HC_CUDA(fn(a, b->sched.tile, grid, b->stream));
+      if (a.q_out != out_of(s))
+        HC_CUDA(cudaMemcpyAsync(out_of(s), a.q_out, 4 * b->ncell * sizeof(R), cudaMemcpyDeviceToDevice, b->stream));
       b->launches += 1;
     }
   }
@@ -199,8 +202,10 @@ template <class R> int per_instance_step(hc_batch* b) {
         b->launches += 2;
       } else {
         a.mode = global ? MODE_FUSED_GLOBAL : MODE_FUSED_LOCAL;
-        a.q_out = out_of(s);
+        a.q_out = out_of(s) == a.q ? qp(1) : out_of(s);
         HC_CUDA(fn(a, b->sched.tile, b->stream));
+        if (a.q_out != out_of(s))
+          HC_CUDA(cudaMemcpyAsync(out_of(s), a.q_out, 4 * b->icells(k) * sizeof(R), cudaMemcpyDeviceToDevice, b->stream));
         b->launches += 1;
       }
     }
